@@ -162,13 +162,37 @@ int check_spheres(lbm_sim *h, const lbm_sphere *sp, int ns) {
 int upload_plan(lbm_sim *h) {
   // pageable source: the copy is staged before cudaMemcpyAsync returns, so the
   // host plan can be rewritten for the next call right away
-  CK(copy_async(h, h->dPlan, &h->hPlan, sizeof(Plan), cudaMemcpyHostToDevice, h->stream));
+  h->planOfStep = false;
+  CK(copy_async(h, h->plan(), &h->hPlan, sizeof(Plan), cudaMemcpyHostToDevice, h->stream));
   return LBM_OK;
 }
 
-// Fill the plan's solid set; when `targets` is true also lay out and clear the
-// per-sphere impulse arrays.
-int set_solids(lbm_sim *h, const lbm_sphere *sp, int ns, bool targets) {
+// The spheres' work arrays, in doubles: impulse slots and the partials of their
+// sums, grown on the handle's stream.
+int ensure_work(lbm_sim *h, long long slots, long long partials) {
+  const struct {
+    double **p;
+    long long *cap, need;
+  } arr[] = {{&h->impAcc, &h->impCap, slots}, {&h->partials, &h->partialsCap, partials}};
+  for (const auto &a : arr) {
+    if (a.need <= *a.cap) continue;
+    if (*a.p) {
+      cudaFreeAsync(*a.p, h->stream);
+      h->deviceBytes -= *a.cap * sizeof(double);
+      *a.p = nullptr;
+      *a.cap = 0;
+    }
+    const long long cap = a.need + a.need / 2;
+    DALLOC(*a.p, cap * sizeof(double));
+    *a.cap = cap;
+  }
+  return LBM_OK;
+}
+
+// Fill the plan's solid set; when `targets` is true also lay out the spheres'
+// impulse slots (clear: they start at zero, for the phase-by-phase hydro
+// stream, which adds to them).
+int set_solids(lbm_sim *h, const lbm_sphere *sp, int ns, bool targets, bool clear = false) {
   SolidSet &ss = h->hPlan.ss;
   memset(&ss, 0, sizeof(ss));
   ss.nsph = ns;
@@ -196,7 +220,7 @@ int set_solids(lbm_sim *h, const lbm_sphere *sp, int ns, bool targets) {
     d.wz = sp[b].wz;
     if (!targets) continue;
     Box bx = box_grow(sphere_box(d.cx, d.cy, d.cz, d.r, h->nx, h->ny, h->nz), 1, h->nx, h->ny, h->nz);
-    if (h->slab) {  // links of cells outside the owned planes belong to the neighbour
+    if (h->slab && clear) {  // links of cells outside the owned planes belong to the neighbour
       bx.lo[2] = std::max(bx.lo[2], h->ownLo);
       bx.hi[2] = std::min(bx.hi[2], h->ownHi);
     }
@@ -219,30 +243,11 @@ int set_solids(lbm_sim *h, const lbm_sphere *sp, int ns, bool targets) {
   h->hPlan.impDoubles = off * 6;
   h->hPlan.redChunks = maxChunks;
   if (!targets) return LBM_OK;
-  long long need = std::max(1LL, off * 6);
-  if (need > h->impCap) {
-    if (h->impAcc) {
-      cudaFreeAsync(h->impAcc, h->stream);
-      h->deviceBytes -= h->impCap * sizeof(double);
-      h->impAcc = nullptr;
-    }
-    long long cap = need + need / 2;
-    DALLOC(h->impAcc, cap * sizeof(double));
-    h->impCap = cap;
-  }
-  long long pneed = (long long)std::max(ns, 1) * maxChunks * 6;
-  if (pneed > h->partialsCap) {
-    if (h->partials) {
-      cudaFreeAsync(h->partials, h->stream);
-      h->deviceBytes -= h->partialsCap * sizeof(double);
-      h->partials = nullptr;
-    }
-    DALLOC(h->partials, pneed * sizeof(double));
-    h->partialsCap = pneed;
-  }
+  int rc = ensure_work(h, std::max(1LL, off * 6), (long long)std::max(ns, 1) * maxChunks * 6);
+  if (rc) return rc;
   h->partialsChunks = maxChunks;
   for (int b = 0; b < ns; b++) ss.imp[b].acc = h->impAcc + offs[b] * 6;
-  if (off > 0) CK(cudaMemsetAsync(h->impAcc, 0, off * 6 * sizeof(double), h->stream));
+  if (clear && off > 0) CK(cudaMemsetAsync(h->impAcc, 0, off * 6 * sizeof(double), h->stream));
   return LBM_OK;
 }
 
@@ -250,7 +255,7 @@ int reduce_impulses(lbm_sim *h, double *d_out) {
   int ns = h->hPlan.ss.nsph;
   if (ns == 0) return LBM_OK;
   dim3 g1(h->partialsChunks, ns);
-  k_impulse_reduce<<<g1, RED_THREADS, 0, h->stream>>>(&h->dPlan->ss, h->partials, h->partialsChunks, d_out,
+  k_impulse_reduce<<<g1, RED_THREADS, 0, h->stream>>>(&h->plan()->ss, h->partials, h->partialsChunks, d_out,
                                                       h->redTickets);
   h->launches++;
   CKL("impulse reduction");
@@ -259,34 +264,27 @@ int reduce_impulses(lbm_sim *h, double *d_out) {
 
 int ensure_counts(lbm_sim *h, long long nch) {
   if (nch <= h->countsCap) return LBM_OK;
-  if (h->counts) {
-    cudaFreeAsync(h->counts, h->stream);
-    h->deviceBytes -= h->countsCap * sizeof(int2);
-    h->counts = nullptr;
-  }
-  DALLOC(h->counts, nch * sizeof(int2));
-  h->countsCap = nch;
+  const size_t bits = SETS_WORDS * 2 * sizeof(uint32_t);
+  for (void *p : {(void *)h->counts, h->setBits})
+    if (p) cudaFreeAsync(p, h->stream);
+  h->deviceBytes -= h->countsCap * (sizeof(int2) + bits);
+  h->counts = nullptr;
+  h->setBits = nullptr;
+  h->countsCap = 0;
+  const long long cap = nch + nch / 2;
+  DALLOC(h->counts, cap * sizeof(int2));
+  DALLOC(h->setBits, cap * bits);
+  h->countsCap = cap;
   return LBM_OK;
 }
 
-// Launch the fresh / dead compaction over the plan's box U (already on the
-// device); maxChunks bounds the plan's chunk count.
-int launch_compaction(lbm_sim *h, long long maxChunks) {
-  if (maxChunks <= 0) {
-    CK(cudaMemsetAsync(h->totals, 0, 2 * sizeof(int), h->stream));
-    h->listsValid = true;
-    return LBM_OK;
-  }
-  int rc = ensure_counts(h, maxChunks);
+// Retag (retag), fresh / dead lists and fresh fill (fill) over the plan's box U
+// (already on the device); maxChunks bounds the plan's chunk count.
+int launch_sets(lbm_sim *h, long long maxChunks, bool retag, bool fill) {
+  int rc = ensure_counts(h, std::max(1LL, maxChunks));
   if (rc) return rc;
-  const unsigned ctas = (unsigned)std::min<long long>(maxChunks, SWEEP_CTAS);
-  k_compact_count<<<ctas, COMPACT_THREADS, 0, h->stream>>>(h->tag, h->tagPrev, h->nx, h->ny, h->dPlan,
-                                                           h->counts);
-  k_compact_scan<<<1, 1024, 0, h->stream>>>(h->counts, h->dPlan, h->totals);
-  k_compact_emit<<<ctas, COMPACT_THREADS, 0, h->stream>>>(h->tag, h->tagPrev, h->nx, h->ny, h->dPlan,
-                                                          h->counts, h->fresh, h->dead, (int)h->listCap);
-  h->launches += 3;
-  CKL("fresh/dead compaction");
+  h->ops->sets(h, maxChunks, retag, fill);
+  CKL("retag, fresh / dead sets");
   h->listsValid = true;
   return LBM_OK;
 }
@@ -316,12 +314,12 @@ void set_box(lbm_sim *h, const Box &bx) {
   h->hPlan.nchunks = (int)((h->hPlan.ucells + COMPACT_CHUNK - 1) / COMPACT_CHUNK);
 }
 
-// fresh / dead lists over a box, scan order
-int compact_sets(lbm_sim *h, const Box &bx) {
+// fresh / dead lists over a box, scan order, and the fresh fill (fill)
+int compact_sets(lbm_sim *h, const Box &bx, bool fill) {
   set_box(h, bx);
   int rc = upload_plan(h);
   if (rc) return rc;
-  return launch_compaction(h, h->hPlan.nchunks);
+  return launch_sets(h, h->hPlan.nchunks, false, fill);
 }
 
 void shift_boxes(lbm_sim *h, const Box &now) {
@@ -499,7 +497,7 @@ void free_all(lbm_sim *h) {
                   h->grad[2], h->grad[3], h->us[0], h->us[1], h->us[2], h->bf[0], h->bf[1],
                   h->bf[2], h->fresh, h->dead, h->counts, h->totals, h->impAcc, h->partials,
                   h->dOut, h->dSph, h->staging, h->dPhiCol, h->dPlan, h->dWatch, h->linkChunks,
-                  h->linkBuf, h->redTickets, h->meshTri, h->dMaps};
+                  h->linkBuf, h->redTickets, h->meshTri, h->dMaps, h->setBits};
   for (void *p : ptrs)
     if (p) cudaFreeAsync(p, h->stream);
   for (int c = 0; c < 2; c++)
@@ -527,13 +525,12 @@ void free_all(lbm_sim *h) {
 
 // ---------------------------------------------------------------- device-resident coupled step
 // One coupled step (sim.step, absorbDeadCells, RigidSphere.step; src/worker.js:96-100)
-// entirely on the device: the plan is computed by k_plan from the device sphere
-// state, so no host round trip is needed between steps.  Split into the parts a
-// batch launches around its shared fused kernel.
-struct CoupledCtx {
-  int ns = 0;
-  long long slotCells = 0, maxU = 0, maxChunks = 0;
-  int redChunks = 0;
+// entirely on the device, as three launches: the retag, the fresh / dead sets
+// and the fresh fill; the fused step; the shells, which also step the spheres
+// and plan the next step from the device sphere state, so no host round trip is
+// needed between steps.
+struct CoupledCtx : StepCtx {
+  long long maxChunks = 0;
 };
 
 // Capacities for the device-computed plan, the plan's history and the device
@@ -556,28 +553,10 @@ int coupled_prepare(lbm_sim *h, const lbm_sphere *sp, int ns, bool frames, Coupl
   if (ns == 0) c.maxU = (h->fullRetagSteps > 0) ? h->n : box_cells(box_union(h->boxLast, h->boxLastLast));
   c.maxChunks = (c.maxU + COMPACT_CHUNK - 1) / COMPACT_CHUNK;
   c.redChunks = (int)((c.slotCells + RED_CHUNK - 1) / RED_CHUNK);
-  long long need = std::max(1LL, (long long)ns * c.slotCells * 6);
-  if (need > h->impCap) {
-    if (h->impAcc) {
-      cudaFreeAsync(h->impAcc, h->stream);
-      h->deviceBytes -= h->impCap * sizeof(double);
-      h->impAcc = nullptr;
-    }
-    DALLOC(h->impAcc, need * sizeof(double));
-    h->impCap = need;
-  }
-  // the slots start at zero; every step's reduction zeroes the slots it reads
-  CK(cudaMemsetAsync(h->impAcc, 0, need * sizeof(double), h->stream));
-  long long pneed = (long long)std::max(ns, 1) * c.redChunks * 6;
-  if (pneed > h->partialsCap) {
-    if (h->partials) {
-      cudaFreeAsync(h->partials, h->stream);
-      h->deviceBytes -= h->partialsCap * sizeof(double);
-      h->partials = nullptr;
-    }
-    DALLOC(h->partials, pneed * sizeof(double));
-    h->partialsCap = pneed;
-  }
+  c.tail = true;
+  if ((rc = ensure_work(h, std::max(1LL, (long long)ns * c.slotCells * 6),
+                        (long long)std::max(ns, 1) * c.redChunks * 6)))
+    return rc;
   h->partialsChunks = c.redChunks;
   if ((rc = ensure_counts(h, std::max(1LL, c.maxChunks)))) return rc;
   if (frames && (rc = ensure_staging(h, (size_t)h->n * 2))) return rc;
@@ -594,31 +573,12 @@ int coupled_prepare(lbm_sim *h, const lbm_sphere *sp, int ns, bool frames, Coupl
   return LBM_OK;
 }
 
-// plan, retag, fresh / dead compaction, fresh fill, impulse slot clearing
-int coupled_pre(lbm_sim *h, const CoupledCtx &c) {
-  k_plan<<<1, 1, 0, h->stream>>>(h->dPlan, h->dSph, c.ns, h->nx, h->ny, h->nz, h->impAcc, c.slotCells,
-                                 c.maxU);
+// the first step's plan (every later one is made by the step before it)
+int coupled_plan(lbm_sim *h, const CoupledCtx &c) {
+  k_plan<<<1, 32, 0, h->stream>>>(h->plan(), h->dSph, c.ns, h->nx, h->ny, h->nz, h->impAcc, c.slotCells,
+                                  c.maxU);
   h->launches++;
-  h->ops->retag_box(h, c.maxU);
-  int rc = launch_compaction(h, c.maxChunks);
-  if (rc) return rc;
-  h->ops->fresh_fill(h);
-  CKL("coupled step (before the fused kernel)");
-  return LBM_OK;
-}
-
-// impulse reduction, dead-cell absorption, RigidSphere.step on the device
-int coupled_post(lbm_sim *h, const CoupledCtx &c) {
-  if (c.ns > 0) {
-    double *dFluid = h->dOut, *dDead = h->dOut + LBM_MAX_SPHERES * 6;
-    dim3 g1(c.redChunks, c.ns);
-    k_impulse_reduce<<<g1, RED_THREADS, 0, h->stream>>>(&h->dPlan->ss, h->partials, c.redChunks, dFluid,
-                                                        h->redTickets);
-    h->ops->absorb_dead(h, dDead);
-    h->ops->sphere_step_device(h, h->dSph, c.ns, h->params.gravity, dFluid, dDead);
-    h->launches++;
-  }
-  CKL("coupled step (after the fused kernel)");
+  CKL("step plan");
   return LBM_OK;
 }
 
@@ -632,9 +592,11 @@ int coupled_frame(lbm_sim *h, uint8_t *dst, bool fused = false) {
   return LBM_OK;
 }
 
-// sphere state and plan history back to the host
-int coupled_finish(lbm_sim *h, lbm_sphere *sp, int ns) {
-  CK(copy_async(h, &h->hPlan, h->dPlan, sizeof(Plan), cudaMemcpyDeviceToHost, h->stream));
+// sphere state and the plan of the last step (of none: the uploaded history)
+// back to the host
+int coupled_finish(lbm_sim *h, lbm_sphere *sp, int ns, int nsteps) {
+  CK(copy_async(h, &h->hPlan, h->dPlan + (nsteps > 0 ? 1 - h->cur : h->cur), sizeof(Plan), cudaMemcpyDeviceToHost,
+                h->stream));
   if (ns > 0)
     CK(copy_async(h, sp, h->dSph, ns * sizeof(lbm_sphere), cudaMemcpyDeviceToHost, h->stream));
   if (int rc = sync_status(h)) return rc;
@@ -774,11 +736,11 @@ int lbm_create(int nx, int ny, int nz, int storage, int device, lbm_sim **out) {
     DALLOC(h->totals, 3 * sizeof(int));
     CK(cudaMemsetAsync(h->totals, 0, 3 * sizeof(int), h->stream));
     DALLOC(h->dOut, 2 * LBM_MAX_SPHERES * 6 * sizeof(double));
-    DALLOC(h->redTickets, LBM_MAX_SPHERES * sizeof(unsigned));
-    CK(cudaMemsetAsync(h->redTickets, 0, LBM_MAX_SPHERES * sizeof(unsigned), h->stream));
+    DALLOC(h->redTickets, (LBM_MAX_SPHERES + 1) * sizeof(unsigned));
+    CK(cudaMemsetAsync(h->redTickets, 0, (LBM_MAX_SPHERES + 1) * sizeof(unsigned), h->stream));
     DALLOC(h->dSph, LBM_MAX_SPHERES * sizeof(lbm_sphere));
-    DALLOC(h->dPlan, sizeof(Plan));
-    CK(cudaMemsetAsync(h->dPlan, 0, sizeof(Plan), h->stream));
+    DALLOC(h->dPlan, 2 * sizeof(Plan));
+    CK(cudaMemsetAsync(h->dPlan, 0, 2 * sizeof(Plan), h->stream));
     DALLOC(h->dPhiCol, (size_t)ny * sizeof(double));
     CK(cudaMallocHost((void **)&h->hOut, 2 * LBM_MAX_SPHERES * 6 * sizeof(double)));
     CK(cudaMallocHost((void **)&h->hTotals, 3 * sizeof(int)));
@@ -1259,10 +1221,7 @@ int lbm_handle_fresh_cells(lbm_sim *h) {
   EntryGuard g(h);
   int rc = need_phases(h);
   if (rc) return rc;
-  if ((rc = compact_sets(h, h->lastRetagBox))) return rc;
-  h->ops->fresh_fill(h);
-  CKL("fresh cells");
-  return LBM_OK;
+  return compact_sets(h, h->lastRetagBox, true);
 }
 
 int lbm_compute_phi_gradients(lbm_sim *h) {
@@ -1311,7 +1270,7 @@ int lbm_stream_hydro_and_macro(lbm_sim *h, const lbm_sphere *sp, int ns, lbm_imp
   if (rc) return rc;
   EntryGuard g(h);
   if ((rc = need_phases(h))) return rc;
-  if ((rc = set_solids(h, sp, ns, true))) return rc;
+  if ((rc = set_solids(h, sp, ns, true, true))) return rc;
   if ((rc = upload_plan(h))) return rc;
   h->ops->stream_hydro_macro(h);
   CKL("streamHydroAndMacro");
@@ -1352,12 +1311,9 @@ int lbm_step_begin(lbm_sim *h, const lbm_sphere *sp, int ns) {
   h->hPlan.boxLast = h->boxLast;
   h->hPlan.boxLastLast = h->boxLastLast;
   if ((rc = upload_plan(h))) return rc;
-  h->ops->retag_box(h, h->hPlan.ucells);
-  CKL("retag box");
   h->lastRetagBox = U;
-  if ((rc = launch_compaction(h, h->hPlan.nchunks))) return rc;
-  h->ops->fresh_fill(h);
-  CKL("fresh cells");
+  if ((rc = launch_sets(h, h->hPlan.nchunks, true, true))) return rc;
+  h->planOfStep = true;
   h->stepNow = now;
   h->stepBegunNs = ns;
   return LBM_OK;
@@ -1378,23 +1334,31 @@ int lbm_step_end(lbm_sim *h, const lbm_sphere *sp, int ns, lbm_impulse *out) {
     if ((rc = lbm_collide_hydro(h))) return rc;
     return lbm_stream_hydro_and_macro(h, sp, ns, out);
   }
+  if (!h->planOfStep) {  // another call has put its own plan in place since the step began
+    if ((rc = set_solids(h, sp, ns, true))) return rc;
+    set_box(h, h->lastRetagBox);
+    if ((rc = upload_plan(h))) return rc;
+  }
   launch_fused(h);
   CKL("fused step");
   if ((rc = flush_frame_copy(h))) return rc;
-  if ((rc = reduce_impulses(h, h->dOut))) return rc;
+  if (ns > 0) {
+    // the shell launch also computes absorbDeadCells, which follows every step
+    // (src/worker.js:96-100) and reads only this step's dead list and values
+    // that the step leaves alone: fetched with the step's impulses below, so
+    // lbm_absorb_dead_cells needs no launch and no wait of its own
+    StepCtx c;
+    c.ns = ns;
+    c.redChunks = h->partialsChunks;
+    h->ops->shell(h, c);
+    CKL("shells");
+  }
   h->cur = 1 - h->cur;
   shift_boxes(h, h->stepNow);
   h->deadAhead.valid = false;
-  if (ns > 0 && out && h->listsValid) {
-    // absorbDeadCells follows every step (src/worker.js:96-100) and reads
-    // only the new half and this step's dead list with the same spheres:
-    // run it now on the step's plan and fetch it with the step's impulses,
-    // so lbm_absorb_dead_cells needs no launch and no wait of its own
-    double *d = h->dOut + LBM_MAX_SPHERES * 6;
-    h->ops->absorb_dead(h, d);
-    CKL("absorbDeadCells");
-    CK(copy_async(h, h->hOut + LBM_MAX_SPHERES * 6, d, (size_t)ns * 6 * sizeof(double), cudaMemcpyDeviceToHost,
-                  h->stream));
+  if (ns > 0 && out) {
+    CK(copy_async(h, h->hOut + LBM_MAX_SPHERES * 6, h->dOut + LBM_MAX_SPHERES * 6, (size_t)ns * 6 * sizeof(double),
+                  cudaMemcpyDeviceToHost, h->stream));
     if ((rc = fetch_out(h, h->dOut, ns, out))) return rc;
     auto &A = h->deadAhead;
     A.ns = ns;
@@ -1455,7 +1419,7 @@ int lbm_absorb_dead_cells(lbm_sim *h, const lbm_sphere *sp, int ns, lbm_impulse 
   if (ns == 0) return LBM_OK;
   if (dead_ahead_take(h, sp, ns, out)) return LBM_OK;
   EntryGuard g(h);
-  if (!h->listsValid && (rc = compact_sets(h, h->lastRetagBox))) return rc;
+  if (!h->listsValid && (rc = compact_sets(h, h->lastRetagBox, false))) return rc;
   if ((rc = set_solids(h, sp, ns, false))) return rc;
   if ((rc = upload_plan(h))) return rc;
   double *d = h->dOut + LBM_MAX_SPHERES * 6;
@@ -1590,21 +1554,26 @@ int lbm_run_coupled(lbm_sim *h, lbm_sphere *sp, int ns, int nsteps, int frame_ev
   int rc = coupled_prepare(h, sp, ns, frame_every > 0 && frames, c);
   if (rc) return rc;
   long long frame = 0;
+  if (nsteps > 0 && (rc = coupled_plan(h, c))) return rc;
+  // without spheres the sets stay empty once the boxes of earlier ones and
+  // pending whole-grid retags are worked off (and both plans say so)
+  const int sparse = ns > 0 ? nsteps : 4;
   for (int s = 0; s < nsteps; s++) {
     const bool frameStep = frame_every > 0 && frames && (s + 1) % frame_every == 0;
-    if ((rc = coupled_pre(h, c))) return rc;
+    if (s < sparse && (rc = launch_sets(h, c.maxChunks, true, true))) return rc;
     // a frame step's fused kernel also writes the step's RG8 volume
     h->fusePack = frameStep ? (uint8_t *)h->staging : nullptr;
     launch_fused(h);
     h->fusePack = nullptr;
-    if ((rc = coupled_post(h, c))) return rc;
+    if (s < sparse) h->ops->shell(h, c);
+    CKL("coupled step");
     h->cur = 1 - h->cur;
     if (frameStep) {
       if ((rc = coupled_frame(h, frames + frame * 2 * h->n, true))) return rc;
       frame++;
     }
   }
-  if ((rc = coupled_finish(h, sp, ns))) return rc;
+  if ((rc = coupled_finish(h, sp, ns, nsteps))) return rc;
   return watch_after(h, nsteps);
 }
 
@@ -1844,7 +1813,7 @@ struct lbm_batch {
   std::vector<cudaEvent_t> joins;
   void *dArgs = nullptr;  // [2][n] descriptors (FusedArgs of the storage type)
   size_t argsCap = 0;
-  void *dSmall = nullptr;  // [2][n] arguments of the batched sparse kernels
+  void *dSmall = nullptr;  // [2][n] arguments of the batched sparse kernels: sets, then shells
   size_t smallCap = 0;
   int *dTileStart = nullptr;  // [n + 1]
   int3 *dTileGrid = nullptr;  // [n]
@@ -2054,22 +2023,25 @@ int lbm_batch_run(lbm_batch *b, lbm_sphere *const *spheres, const int *nspheres,
                                      ctx[s]));
   int rc = batch_tables(b);
   if (rc) return rc;
-  // the sparse kernels' arguments of every scene for both parities, and the
-  // batched launches' grids (sized for the largest scene's plan bounds)
-  const size_t sb = ops->small_args_bytes();
-  std::vector<unsigned char> small(2 * (size_t)n * sb);
-  unsigned retagCtas = 1, compactCtas = 1;
+  // the sparse kernels' arguments of every scene for both parities, and their
+  // grids: for the sets, blocks for the largest scene's box, but no more in all
+  // than fill the device a few times (a scene's blocks stride over its box)
+  const size_t sb = ops->small_args_bytes(), hb = ops->shell_args_bytes(), shellOff = 2 * (size_t)n * sb;
+  std::vector<unsigned char> small(shellOff + 2 * (size_t)n * hb);
+  long long maxChunks = 1;
   int redX = 1, nsMax = 0;
   for (int s = 0; s < n; s++) {
     lbm_sim *h = b->sims[s];
-    for (int p = 0; p < 2; p++)
-      ops->small_args(h, h->cur ^ p, ctx[s].ns, ctx[s].slotCells, ctx[s].maxU, ctx[s].redChunks,
-                      &small[((size_t)p * n + s) * sb]);
-    retagCtas = std::max(retagCtas, std::min(nblocks(std::max(1LL, ctx[s].maxU), 256), SWEEP_CTAS));
-    compactCtas = std::max(compactCtas, (unsigned)std::min<long long>(std::max(1LL, ctx[s].maxChunks), SWEEP_CTAS));
+    for (int p = 0; p < 2; p++) {
+      ops->small_args(h, h->cur ^ p, &small[((size_t)p * n + s) * sb]);
+      ops->shell_args(h, ctx[s], h->cur ^ p, &small[shellOff + ((size_t)p * n + s) * hb]);
+    }
+    maxChunks = std::max(maxChunks, ctx[s].maxChunks);
     redX = std::max(redX, ctx[s].redChunks);
     nsMax = std::max(nsMax, ctx[s].ns);
   }
+  const unsigned setCtas =
+      (unsigned)std::min<long long>(maxChunks, std::max<long long>(8, 4LL * SWEEP_CTAS / n));
   if (small.size() > b->smallCap) {
     if (b->dSmall) cudaFreeAsync(b->dSmall, b->origin);
     b->dSmall = nullptr;
@@ -2078,8 +2050,7 @@ int lbm_batch_run(lbm_batch *b, lbm_sphere *const *spheres, const int *nspheres,
   }
   BCK(cudaMemcpyAsync(b->dSmall, small.data(), small.size(), cudaMemcpyHostToDevice, b->origin));
   BCK(cudaStreamSynchronize(b->origin));  // the host vector goes out of scope
-  const int tiles = batch_tiles(b);
-  const int ctas = std::min(tiles, ops->fused_batch_ctas(launch_shape(b, b->rows), b->device));
+  const int ctas = std::min(batch_tiles(b), ops->fused_batch_ctas(launch_shape(b, b->rows), b->device));
   const size_t ab = ops->fused_args_bytes();
 
   // Graph mode replays a captured chunk of 2 steps (the ping-pong halves
@@ -2101,12 +2072,12 @@ int lbm_batch_run(lbm_batch *b, lbm_sphere *const *spheres, const int *nspheres,
   // scenes, around the shared fused launch, all on the batch's stream
   auto emit_step = [&](int parity) -> int {
     const void *A = (const unsigned char *)b->dSmall + (size_t)parity * n * sb;
-    ops->batch_pre(A, n, retagCtas, compactCtas, b->origin);
+    ops->batch_sets(A, n, setCtas, b->origin);
     BCK(cudaGetLastError());
     ops->fused_batch((const unsigned char *)b->dArgs + (size_t)parity * n * ab, b->dTileStart, b->dTileGrid,
                      n, launch_shape(b, b->rows), ctas, b->origin);
     BCK(cudaGetLastError());
-    ops->batch_post(A, n, redX, nsMax, b->origin);
+    ops->batch_shell((const unsigned char *)b->dSmall + shellOff + (size_t)parity * n * hb, n, redX, nsMax, b->origin);
     BCK(cudaGetLastError());
     for (int s = 0; s < n; s++) b->sims[s]->cur ^= 1;
     return LBM_OK;
@@ -2133,7 +2104,7 @@ int lbm_batch_run(lbm_batch *b, lbm_sphere *const *spheres, const int *nspheres,
   if (graph) {
     std::vector<long long> key = {b->rows, b->zchunk, (long long)(uintptr_t)b->dArgs,
                                   (long long)(uintptr_t)b->dTileStart, ctas, (long long)(uintptr_t)b->dSmall,
-                                  retagCtas, compactCtas, redX, nsMax};
+                                  setCtas, redX, nsMax};
     for (int s = 0; s < n; s++) {
       lbm_sim *h = b->sims[s];
       const long long v[] = {(long long)(uintptr_t)h,           h->cur,      ctx[s].ns,
@@ -2173,6 +2144,10 @@ int lbm_batch_run(lbm_batch *b, lbm_sphere *const *spheres, const int *nspheres,
     }
   }
 
+  if (nsteps > 0) {
+    ops->batch_plan((const unsigned char *)b->dSmall + shellOff, n, b->origin);
+    BCK(cudaGetLastError());
+  }
   long long done = 0;
   while (done < nsteps) {
     if (graph && nsteps - done >= 2) {
@@ -2189,7 +2164,7 @@ int lbm_batch_run(lbm_batch *b, lbm_sphere *const *spheres, const int *nspheres,
   }
   BCK(cudaStreamSynchronize(b->origin));
   for (int s = 0; s < n; s++)
-    BSIM(b->sims[s], coupled_finish(b->sims[s], nspheres[s] ? spheres[s] : nullptr, nspheres[s]));
+    BSIM(b->sims[s], coupled_finish(b->sims[s], nspheres[s] ? spheres[s] : nullptr, nspheres[s], nsteps));
   // every scene's watchdog advances and scans; the first scene that reports
   // gives the batch's status and message
   int first = LBM_OK;

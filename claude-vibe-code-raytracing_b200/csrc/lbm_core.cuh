@@ -354,10 +354,10 @@ __host__ __device__ inline long long box_cells(const Box &b) {
   return (long long)(b.hi[0] - b.lo[0] + 1) * (b.hi[1] - b.lo[1] + 1) * (b.hi[2] - b.lo[2] + 1);
 }
 
-// Impulse accumulation target of one sphere: a dense array of 6 doubles per
-// cell over the sphere's bounding box grown by one cell.  Each fluid cell's
-// slot is written only by the thread that owns the cell, so the result does not
-// depend on tiling or scheduling; a fixed-order reduction sums it.
+// Impulse slots of one sphere: six doubles per cell over the sphere's bounding
+// box grown by one cell, where every cell with a link to the sphere lies.  Each
+// cell's slot is written only by the thread that computes the cell, so a
+// fixed-order sum does not depend on tiling or scheduling.
 struct ImpulseTarget {
   double *acc;  // [cells][6]
   int lo[3], dim[3];
@@ -365,17 +365,19 @@ struct ImpulseTarget {
 
 struct SolidSet {
   int nsph;
-  // z slab: dead cells outside local planes [zlo, zend) give no impulse (their
+  // z slab: cells outside local planes [zlo, zend) give no impulse (their
   // slab's neighbour owns them); zend = 0 (the default) means no limit
   int zlo, zend;
   SphereDesc sph[LBM_MAX_SPHERES];
   ImpulseTarget imp[LBM_MAX_SPHERES];
 };
 
-// Per-step plan of the sparse work around the spheres, in device memory.  The
-// host-driven API computes it on the host and copies it up; the device-resident
-// loop computes it with k_plan from the device copy of the sphere state.  Every
-// kernel of a step reads it, so launch grids can be sized by upper bounds.
+// Per-step plan of the sparse work around the spheres, in device memory: two
+// of them, the step that reads population half c uses plan c.  The host-driven
+// API computes the plan on the host; in the device-resident loop each step's
+// shell launch computes the next step's from the device copy of the sphere
+// state.  Every kernel of a step reads it, so launch grids can be sized by
+// upper bounds.
 struct Plan {
   SolidSet ss;
   Box U;             // retag / fresh-dead compaction box

@@ -15,10 +15,14 @@
 //   2. after a barrier the cell threads pull plane z from the ring
 //      (streamPhase src/sim.js:376-397, streamHydroAndMacro src/sim.js:509-543):
 //      fluid sources give their post-collision value, wall and solid sources
-//      bounce back the cell's own value, SOLID sources add the Ladd
-//      moving-wall term and FP64 momentum exchange; then the macros
+//      bounce back the cell's own value; then the macros
 //      (src/sim.js:545-576), and the new populations and macros are written
 //      once.
+// The cells next to a sphere are finished by the shell launch that follows
+// (lbm_shell.cuh): it adds the Ladd moving-wall terms of their links to SOLID
+// sources and sums the momentum exchange in FP64.  In this kernel that code,
+// rarely run, made every warp along a sphere wait 10 us a plane and the loop
+// slower everywhere else.
 //
 // The collision is evaluated in the equivalent form
 //   f*_k = (1 - w) f_k + w_k (C0 + e.V + (e.u)(e.Q)),
@@ -61,7 +65,6 @@ struct FusedArgs {
   int cur;
   int zchunk;
   double om, omP, A, beta4, kappa, rhoG, dRho, gravity, sharpC4;
-  const SolidSet *ss;
   int *status;   // set non-zero when a bounded wait of the step runs out
   int withhold;  // test hook: the bulk-staged form does not issue each tile's first copy
   uint8_t *pack; // frame step: the RG8 volume of the step's result (planes 1 .. nz-2), else null
@@ -75,9 +78,6 @@ constexpr int slot27(int k) {
     if (kDir[j][2] == kDir[k][2]) s++;
   return s;
 }
-// the same, indexable at run time
-static __constant__ signed char c_slot27[27] = {0, 1, 2, 3, 4, 0, 0, 5, 6, 7, 8, 1, 1, 2,
-                                                 2, 3, 3, 4, 4, 5, 5, 6, 6, 7, 7, 8, 8};
 // ring plane offsets (in planes of NC values)
 constexpr int RING_F_M = 0, RING_F_Z = 18, RING_F_P = 36;  // 2x9, 2x9, 3x9
 constexpr int RING_H_M = 63, RING_H_Z = 65, RING_H_P = 75;  // 2x1, 2x5, 3x1
@@ -407,14 +407,14 @@ __device__ __forceinline__ Real edot(Real X, Real Y, Real Z) {
 // tile cell; opposite pairs evaluated together); MODE 1: the directions of the
 // compile-time halo side (SX, SY); MODE 2: every direction, one at a time (a
 // halo cell whose side is known at run time).  Returns gradient, laplacian
-// and phi of the cell.  Every operation rounds explicitly (rmul / radd / rsub
+// and   Every operation rounds explicitly (rmul / radd / rsub
 // / rfma), so a tile cell and a halo cell of another tile get the same bits
 // whatever the compiler would contract in either context.
 template <class PopT, int MODE, int SX, int SY>
 __device__ __forceinline__ void collide_cell(const CollK<typename Prec<PopT>::Real> &K, const CellLoad<PopT> &L,
                                              CellOut<PopT> &o, typename Prec<PopT>::Real &ogx,
                                              typename Prec<PopT>::Real &ogy, typename Prec<PopT>::Real &ogz,
-                                             typename Prec<PopT>::Real &olap, typename Prec<PopT>::Real &ophi) {
+                                             typename Prec<PopT>::Real &olap) {
   using Real = typename Prec<PopT>::Real;
   using C = Codec<PopT>;
   if constexpr (MODE == 1 && SY < 0) o.tg2 = L.tg;
@@ -483,7 +483,32 @@ __device__ __forceinline__ void collide_cell(const CollK<typename Prec<PopT>::Re
   ogy = gyv;
   ogz = gzv;
   olap = lap;
-  ophi = p;
+}
+
+// A cell's macros from its streamed sums (src/sim.js:545-576): rhoA and m the
+// populations' sums, p the new phi, gradients and laplacian of the old one.
+// Explicitly rounded like the collision, so every kernel that finishes a cell
+// gives the same bits.
+template <class Real>
+__device__ __forceinline__ void finish_macros(const CollK<Real> &K, Real p, Real gx, Real gy, Real gz, Real lap,
+                                              Real rhoA, Real mx, Real my, Real mz, Real &rhoN, Real &ux, Real &uy,
+                                              Real &uz) {
+  const Real one = (Real)1, half = (Real)0.5;
+  rhoN = rhoA > (Real)0.01 ? rhoA : (Real)0.01;
+  const Real rhoPhN = rfma(p, K.dRho, K.rhoG);
+  const Real mu = rfma(-K.kappa, lap, rmul(rmul(rmul(K.beta4, p), rsub(p, one)), rfma((Real)2, p, -one)));
+  const Real Fx = rmul(mu, gx), Fy = rfma(mu, gy, rmul(rhoPhN, K.grav)), Fz = rmul(mu, gz);
+  const Real inv = one / rhoPhN;
+  ux = rmul(rfma(half, Fx, mx), inv);
+  uy = rmul(rfma(half, Fy, my), inv);
+  uz = rmul(rfma(half, Fz, mz), inv);
+  const Real u2 = rfma(uz, uz, rfma(uy, uy, rmul(ux, ux)));
+  if (u2 > (Real)(0.2 * 0.2)) {
+    const Real sc = (Real)0.2 / sqrt(u2);
+    ux = rmul(ux, sc);
+    uy = rmul(uy, sc);
+    uz = rmul(uz, sc);
+  }
 }
 
 // One tile (bx, by) of 32 x TY columns over z-chunk bz of one scene.
@@ -503,7 +528,6 @@ __device__ __forceinline__ void fused_tile(const FusedArgs<PopT> &a, int bx, int
   uint8_t *stag = smem_raw + SM::ringBytes;                               // [3][NC]
 
   const auto &s = a.s;
-  const SolidSet &ss = *a.ss;
   const int cur = a.cur, nxt = 1 - cur;
   const PopT *__restrict__ Fc = s.F[cur];
   const PopT *__restrict__ Hc = s.H[cur];
@@ -522,9 +546,6 @@ __device__ __forceinline__ void fused_tile(const FusedArgs<PopT> &a, int bx, int
   constexpr int RING = RING_PLANES * NC, TAGS = 3 * NC;
   constexpr int G27 = PopGroups<Q27>::G, G7 = PopGroups<Q7>::G;
   constexpr int BLK27 = PopGroups<Q27>::BLOCK, BLK7 = PopGroups<Q7>::BLOCK;
-  const Real om = (Real)a.om, omP = (Real)a.omP, A = (Real)a.A;
-  const Real beta4 = (Real)a.beta4, kappa = (Real)a.kappa, rhoG = (Real)a.rhoG;
-  const Real dRho = (Real)a.dRho, grav = (Real)a.gravity, sharpC4 = (Real)a.sharpC4;
 
   const int tx = threadIdx.x, ty = threadIdx.y;
   const bool haloA = ty == TY, haloWarp = ty >= TY;
@@ -652,10 +673,10 @@ __device__ __forceinline__ void fused_tile(const FusedArgs<PopT> &a, int bx, int
 
   // Compute phase: the collision of one cell into registers (o), for emit.
   const CollK<Real> K = coll_consts(a);
-  auto compute = [&](auto MODEc, auto SXc, auto SYc, const LD &L, CO &o, Real &ogx, Real &ogy, Real &ogz, Real &olap,
-                     Real &ophi) __attribute__((always_inline)) {
+  auto compute = [&](auto MODEc, auto SXc, auto SYc, const LD &L, CO &o, Real &ogx, Real &ogy, Real &ogz,
+                     Real &olap) __attribute__((always_inline)) {
     collide_cell<PopT, decltype(MODEc)::value, decltype(SXc)::value, decltype(SYc)::value>(K, L, o, ogx, ogy, ogz,
-                                                                                         olap, ophi);
+                                                                                         olap);
   };
 
   // Collide plane q: cell warps their own cells; halo warp A the rows above
@@ -663,27 +684,27 @@ __device__ __forceinline__ void fused_tile(const FusedArgs<PopT> &a, int bx, int
   // warp B the side columns and corners.
   // (lambdas are forced inline: an outlined closure would live in local memory)
   auto halo_plane = [&](int q, CO &o) __attribute__((always_inline)) {
-    Real d0, d1, d2, d3, d4;
+    Real d0, d1, d2, d3;
     if (haloA) {
       LD top, bot;
       load(IC<1>{}, IC<0>{}, IC<1>{}, 0, 0, true, q, x, y0 - 1, top);
       load(IC<1>{}, IC<0>{}, IC<-1>{}, 0, 0, true, q, x, y0 + TY, bot);
-      compute(IC<1>{}, IC<0>{}, IC<1>{}, top, o, d0, d1, d2, d3, d4);
-      compute(IC<1>{}, IC<0>{}, IC<-1>{}, bot, o, d0, d1, d2, d3, d4);
+      compute(IC<1>{}, IC<0>{}, IC<1>{}, top, o, d0, d1, d2, d3);
+      compute(IC<1>{}, IC<0>{}, IC<-1>{}, bot, o, d0, d1, d2, d3);
     } else {
       LD L;
       load(IC<2>{}, IC<0>{}, IC<0>{}, sideSx, sideSy, sideAct, q, x0 - 1 + sideLx, y0 - 1 + sideLy, L);
-      compute(IC<2>{}, IC<0>{}, IC<0>{}, L, o, d0, d1, d2, d3, d4);
+      compute(IC<2>{}, IC<0>{}, IC<0>{}, L, o, d0, d1, d2, d3);
     }
   };
   // collide plane q into registers (o: a cell warp's cell, halo warp A's two
   // rows, halo warp B's side cell) ...
-  auto collide_plane = [&](int q, CO &o, Real &ogx, Real &ogy, Real &ogz, Real &olap,
-                           Real &ophi) __attribute__((always_inline)) {
+  auto collide_plane = [&](int q, CO &o, Real &ogx, Real &ogy, Real &ogz,
+                           Real &olap) __attribute__((always_inline)) {
     if (!haloWarp) {
       LD L;
       load(IC<0>{}, IC<0>{}, IC<0>{}, 0, 0, true, q, x, y, L);
-      compute(IC<0>{}, IC<0>{}, IC<0>{}, L, o, ogx, ogy, ogz, olap, ophi);
+      compute(IC<0>{}, IC<0>{}, IC<0>{}, L, o, ogx, ogy, ogz, olap);
     } else {
       halo_plane(q, o);
     }
@@ -700,8 +721,8 @@ __device__ __forceinline__ void fused_tile(const FusedArgs<PopT> &a, int bx, int
     }
   };
 
-  Real gxC = 0, gyC = 0, gzC = 0, lapC = 0, phC = 0;
-  Real gxN = 0, gyN = 0, gzN = 0, lapN = 0, phN = 0;
+  Real gxC = 0, gyC = 0, gzC = 0, lapC = 0;
+  Real gxN = 0, gyN = 0, gzN = 0, lapN = 0;
   const bool colActive = !haloWarp && x >= 1 && x <= nx - 2 && y >= 1 && y <= ny - 2;
 
   // Iteration q collides plane q and pulls plane q - 1 (planes zb-1 .. ze are
@@ -710,7 +731,7 @@ __device__ __forceinline__ void fused_tile(const FusedArgs<PopT> &a, int bx, int
   // plane q - 1.
   for (int q = zb - 1; q <= ze; q++) {
     CO o;
-    collide_plane(q, o, gxN, gyN, gzN, lapN, phN);
+    collide_plane(q, o, gxN, gyN, gzN, lapN);
     // plane q's slots of the ring are free once every warp has pulled plane
     // q - 2; a warp that gets here early has its loads and collision of plane
     // q behind it
@@ -761,7 +782,6 @@ __device__ __forceinline__ void fused_tile(const FusedArgs<PopT> &a, int bx, int
       const int obHM = (RING_H_M + (z & 1)) * NC + own;
       const int obHP = (RING_H_P + (z % 3)) * NC + own;
       const int tbM = ((z + 1) % 3) * NC + own, tbZ = sC * NC + own, tbP = ((z + 2) % 3) * NC + own;
-      const Real rhoPhOld = rfma(phC, dRho, rhoG);
       Real rhoA = 0, mx = 0, my = 0, mz = 0, hsum = 0;
       Real hn[Q7];
       Real val4[4], ref4[4];  // the current group's values and offsets, encoded and stored as one vector
@@ -816,54 +836,7 @@ __device__ __forceinline__ void fused_tile(const FusedArgs<PopT> &a, int bx, int
           hsum += hk;
         }
       });
-      // Links to SOLID sources (rare): Ladd moving-wall term
-      // 2 w_k rho_phase(phi_old) (e_k . u_s) / cs^2 and the FP64 momentum
-      // exchange -(f_opp + f_k) e_k at the solid cell (src/sim.js:517-536).
-      static_assert(TAG_FLUID == 0 && (TAG_SOLID & TAG_WALL) == 0, "tag bits");
-      if (orTags & TAG_SOLID) {
-        uint32_t solidM = 0;
-#pragma unroll 1
-        for (int k = 1; k < Q27; k++) {
-          const int ez = dcomp(k, 2);
-          const int tb = ez < 0 ? tbM : (ez == 0 ? tbZ : tbP);
-          const int so = -dcomp(k, 1) * RX - dcomp(k, 0);
-          if (stag[sm_at(tb + so, TAGS, 13)] == TAG_SOLID) solidM |= 1u << k;
-        }
-        double acc[6] = {0, 0, 0, 0, 0, 0};
-        int owner = -1;
-        for (uint32_t m = solidM; m; m &= m - 1) {
-          const int k = __ffs(m) - 1;
-          const int ex = dcomp(k, 0), ey = dcomp(k, 1), ez = dcomp(k, 2);
-          const int o = opp_of(k), oz = -ez;
-          const int sx = x - ex, sy = y - ey, sz = z - ez;
-          const int b = owner_of<LBM_MAX_SPHERES>(ss.sph, ss.nsph, sx, sy, sz);
-          if (b < 0) continue;
-          double ox, oy, oz_;
-          sphere_surface_velocity(ss.sph[b], sx, sy, sz, ox, oy, oz_);
-          // surface velocity rounded as the reference stores it (Float32Array us)
-          const Real eus = (Real)ex * (Real)ox + (Real)ey * (Real)oy + (Real)ez * (Real)oz_;
-          const Real w = (Real)w27_of(k);
-          const Real corr = (Real)2 * w * rhoPhOld * eus * (Real)3;
-          const int obF = oz < 0 ? obFM : (oz == 0 ? sbFZ : obFP);
-          const Real fopp = ring[sm_at(obF + c_slot27[o] * NC, RING, 19)];
-          const Real fk = fopp + corr;
-          st_at(Fn, bF + pofs(k), nF, 15, C::enc(fk, w));
-          rhoA += corr;
-          mx += (Real)ex * corr;
-          my += (Real)ey * corr;
-          mz += (Real)ez * corr;
-          if (b != owner) {
-            flush_impulse(ss, owner, x, y, z, acc);
-            owner = b;
-          }
-          const double mom = __dadd_rn((double)fopp, (double)fk);
-          impulse_terms(ss.sph[b], sx, sy, sz, -mom * ex, -mom * ey, -mom * ez, acc);
-        }
-        flush_impulse(ss, owner, x, y, z, acc);
-      }
-
       // macros (src/sim.js:545-576)
-      const Real rhoN = rhoA > (Real)0.01 ? rhoA : (Real)0.01;
       const Real p = hsum < (Real)0 ? (Real)0 : hsum > (Real)1 ? (Real)1 : hsum;
       static_for<0, Q7>([&](auto KK) {
         constexpr int k = decltype(KK)::value;
@@ -875,23 +848,11 @@ __device__ __forceinline__ void fused_tile(const FusedArgs<PopT> &a, int bx, int
           st4_at(Hn, bH + pofs(k & ~3), nH, 17, enc4);
         }
       });
-      // explicitly rounded like the collision, so every instance of this
-      // kernel (tile shapes, staged or not, batched or not) gives the same bits
-      const Real one = (Real)1, half = (Real)0.5;
-      const Real rhoPhN = rfma(p, dRho, rhoG);
-      const Real mu = rfma(-kappa, lapC, rmul(rmul(rmul(beta4, p), rsub(p, one)), rfma((Real)2, p, -one)));
-      const Real Fx = rmul(mu, gxC), Fy = rfma(mu, gyC, rmul(rhoPhN, grav)), Fz = rmul(mu, gzC);
-      const Real inv = one / rhoPhN;
-      Real uxn = rmul(rfma(half, Fx, mx), inv);
-      Real uyn = rmul(rfma(half, Fy, my), inv);
-      Real uzn = rmul(rfma(half, Fz, mz), inv);
-      const Real u2 = rfma(uzn, uzn, rfma(uyn, uyn, rmul(uxn, uxn)));
-      if (u2 > (Real)(0.2 * 0.2)) {
-        const Real sc = (Real)0.2 / sqrt(u2);
-        uxn = rmul(uxn, sc);
-        uyn = rmul(uyn, sc);
-        uzn = rmul(uzn, sc);
-      }
+      Real rhoN, uxn, uyn, uzn;
+      finish_macros(K, p, gxC, gyC, gzC, lapC, rhoA, mx, my, mz, rhoN, uxn, uyn, uzn);
+      // a cell next to a sphere leaves the sums themselves: the shell launch
+      // adds its moving-wall links and finishes it
+      if (orTags & TAG_SOLID) rhoN = rhoA, uxn = mx, uyn = my, uzn = mz;
       st_at(s.rho[nxt], i, nCell, 18, rhoN);
       st_at(s.phi[nxt], i, nCell, 18, p);
       if constexpr (UPAD) {
@@ -913,7 +874,6 @@ __device__ __forceinline__ void fused_tile(const FusedArgs<PopT> &a, int bx, int
     gyC = gyN;
     gzC = gzN;
     lapC = lapN;
-    phC = phN;
   }
 }
 

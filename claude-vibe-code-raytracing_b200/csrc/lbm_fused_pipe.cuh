@@ -212,7 +212,6 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
   int *abortF = reinterpret_cast<int *>(smem + SM::barOff + 16);
 
   const auto &s = a.s;
-  const SolidSet &ss = *a.ss;
   const int cur = a.cur, nxt = 1 - cur;
   const PopT *__restrict__ Fc = s.F[cur];
   const PopT *__restrict__ Hc = s.H[cur];
@@ -228,8 +227,6 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
   const uint8_t *__restrict__ tagA = s.tag;
   const int nx = s.nx, ny = s.ny, nz = s.nz, nxny = nx * ny;
   const long long nCell = s.n, nF = pop_elems(s.n, Q27), nH = pop_elems(s.n, Q7);
-  const Real kappa = (Real)a.kappa, beta4 = (Real)a.beta4, rhoG = (Real)a.rhoG;
-  const Real dRho = (Real)a.dRho, grav = (Real)a.gravity;
   const CollK<Real> K = coll_consts(a);
 
   const int tx = threadIdx.x, ty = threadIdx.y;
@@ -627,8 +624,8 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
     L.tg = tg;
   };
 
-  Real gxC = 0, gyC = 0, gzC = 0, lapC = 0, phC = 0;
-  Real gxN = 0, gyN = 0, gzN = 0, lapN = 0, phN = 0;
+  Real gxC = 0, gyC = 0, gzC = 0, lapC = 0;
+  Real gxN = 0, gyN = 0, gzN = 0, lapN = 0;
   const bool colActive = cellWarp && x >= 1 && x <= nx - 2 && y >= 1 && y <= ny - 2;
 
   if (producer) {
@@ -682,20 +679,20 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
       } else {
         load(IC<0>{}, IC<0>{}, IC<0>{}, 0, 0, true, q, x, y, L);
       }
-      collide_cell<PopT, 0, 0, 0>(K, L, o, gxN, gyN, gzN, lapN, phN);
+      collide_cell<PopT, 0, 0, 0>(K, L, o, gxN, gyN, gzN, lapN);
     } else {
       // the halo warps load after the barrier that ends the previous plane,
       // while the cell warps pull it: their latency is off the critical path
-      Real d0, d1, d2, d3, d4;
+      Real d0, d1, d2, d3;
       LD Lh, Lh2;
       halo_load(q, Lh, Lh2);
       if (haloRows) {
-        collide_cell<PopT, 1, 0, 1>(K, Lh, o, d0, d1, d2, d3, d4);
-        collide_cell<PopT, 1, 0, -1>(K, Lh2, o, d0, d1, d2, d3, d4);
+        collide_cell<PopT, 1, 0, 1>(K, Lh, o, d0, d1, d2, d3);
+        collide_cell<PopT, 1, 0, -1>(K, Lh2, o, d0, d1, d2, d3);
       } else if (!sideRight) {
-        collide_cell<PopT, 1, 1, 0>(K, Lh, o, d0, d1, d2, d3, d4);
+        collide_cell<PopT, 1, 1, 0>(K, Lh, o, d0, d1, d2, d3);
       } else {
-        collide_cell<PopT, 1, -1, 0>(K, Lh, o, d0, d1, d2, d3, d4);
+        collide_cell<PopT, 1, -1, 0>(K, Lh, o, d0, d1, d2, d3);
       }
     }
     parity ^= 1u;
@@ -779,7 +776,6 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
       const int sHP = R::HP + zPs * R::grp(7, 1);
       const int oHM = R::HM + zMo * R::grp(7, -1), oHP = R::HP + zPo * R::grp(7, 1);
       const int tbM = ring_copy<CT>(z + 1) * NC + own, tbZ = sC * NC + own, tbP = ring_copy<CT>(z - 1) * NC + own;
-      const Real rhoPhOld = rfma(phC, dRho, rhoG);
       Real rhoA = 0, mx = 0, my = 0, mz = 0, hsum = 0;
       Real hn[Q7];
       Real val4[4], ref4[4];
@@ -815,8 +811,7 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
           if constexpr (k == Q27 - 1) val4[3] = ref4[3] = 0;  // pad of the last group: encodes to +0
           C::enc4(val4, ref4, enc4);
           if constexpr (UPAD && k == Q27 - 1) {
-            // the last group waits for ux, its pad (stored at once below
-            // where SOLID links rewrite its elements)
+            // the last group waits for ux, its pad
             lastF[0] = enc4[0], lastF[1] = enc4[1], lastF[2] = enc4[2], lastF[3] = enc4[3];
           } else {
             st4_at(Fn, bF + pofs(k & ~3), nF, 15, enc4);
@@ -842,75 +837,13 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
           hsum += hk;
         }
       });
-      // Links to SOLID sources (rare): Ladd moving-wall term and the FP64
-      // momentum exchange (src/sim.js:517-536), directions from a bit mask.
-      static_assert(TAG_FLUID == 0 && (TAG_SOLID & TAG_WALL) == 0, "tag bits");
-      if (orTags & TAG_SOLID) {
-        if constexpr (UPAD) st4_at(Fn, bF + pofs(Q27 - 3), nF, 15, lastF);  // before the links rewrite it
-        uint32_t solidM = 0;
-#pragma unroll 1
-        for (int k = 1; k < Q27; k++) {
-          const int ez = dcomp(k, 2);
-          const int tb = ez < 0 ? tbM : (ez == 0 ? tbZ : tbP);
-          const int so = -dcomp(k, 1) * RX - dcomp(k, 0);
-          if (stag[sm_at(tb + so, TAGS, 13)] == TAG_SOLID) solidM |= 1u << k;
-        }
-        double acc[6] = {0, 0, 0, 0, 0, 0};
-        int owner = -1;
-        for (uint32_t m = solidM; m; m &= m - 1) {
-          const int k = __ffs(m) - 1;
-          const int ex = dcomp(k, 0), ey = dcomp(k, 1), ez = dcomp(k, 2);
-          const int o = opp_of(k), oz = -ez;
-          const int sx = x - ex, sy = y - ey, sz = z - ez;
-          const int b = owner_of<LBM_MAX_SPHERES>(ss.sph, ss.nsph, sx, sy, sz);
-          if (b < 0) continue;
-          double ox, oy, oz_;
-          sphere_surface_velocity(ss.sph[b], sx, sy, sz, ox, oy, oz_);
-          // surface velocity rounded as the reference stores it (Float32Array us)
-          const Real eus = (Real)ex * (Real)ox + (Real)ey * (Real)oy + (Real)ez * (Real)oz_;
-          const Real w = (Real)w27_of(k);
-          const Real corr = (Real)2 * w * rhoPhOld * eus * (Real)3;
-          // own value of the opposite direction o at (tx, ty) in plane z
-          int oi = oz < 0 ? oFM : (oz == 0 ? sFZ : oFP);
-          static_for<1, Q27>([&](auto KK) {
-            constexpr int kk = decltype(KK)::value;
-            if (kk == o) oi += r33 + R::at(27, kk, 0, 0);
-          });
-          const Real fopp = ring[sm_at(oi, RING, 19)];
-          const Real fk = fopp + corr;
-          st_at(Fn, bF + pofs(k), nF, 15, C::enc(fk, w));
-          rhoA += corr;
-          mx += (Real)ex * corr;
-          my += (Real)ey * corr;
-          mz += (Real)ez * corr;
-          if (b != owner) {
-            flush_impulse(ss, owner, x, y, z, acc);
-            owner = b;
-          }
-          const double mom = __dadd_rn((double)fopp, (double)fk);
-          impulse_terms(ss.sph[b], sx, sy, sz, -mom * ex, -mom * ey, -mom * ez, acc);
-        }
-        flush_impulse(ss, owner, x, y, z, acc);
-      }
-
       // macros (src/sim.js:545-576)
-      const Real rhoN = rhoA > (Real)0.01 ? rhoA : (Real)0.01;
       const Real p = hsum < (Real)0 ? (Real)0 : hsum > (Real)1 ? (Real)1 : hsum;
-      const Real one = (Real)1, half = (Real)0.5;
-      const Real rhoPhN = rfma(p, dRho, rhoG);
-      const Real mu = rfma(-kappa, lapC, rmul(rmul(rmul(beta4, p), rsub(p, one)), rfma((Real)2, p, -one)));
-      const Real Fx = rmul(mu, gxC), Fy = rfma(mu, gyC, rmul(rhoPhN, grav)), Fz = rmul(mu, gzC);
-      const Real inv = one / rhoPhN;
-      Real uxn = rmul(rfma(half, Fx, mx), inv);
-      Real uyn = rmul(rfma(half, Fy, my), inv);
-      Real uzn = rmul(rfma(half, Fz, mz), inv);
-      const Real u2 = rfma(uzn, uzn, rfma(uyn, uyn, rmul(uxn, uxn)));
-      if (u2 > (Real)(0.2 * 0.2)) {
-        const Real sc = (Real)0.2 / sqrt(u2);
-        uxn = rmul(uxn, sc);
-        uyn = rmul(uyn, sc);
-        uzn = rmul(uzn, sc);
-      }
+      Real rhoN, uxn, uyn, uzn;
+      finish_macros(K, p, gxC, gyC, gzC, lapC, rhoA, mx, my, mz, rhoN, uxn, uyn, uzn);
+      // a cell next to a sphere leaves the sums themselves: the shell launch
+      // adds its moving-wall links and finishes it
+      if (orTags & TAG_SOLID) rhoN = rhoA, uxn = mx, uyn = my, uzn = mz;
       // h, the last group's pad holding uy where u sits in the pads (the
       // FP32 / FP64 codec stores it unchanged), +0 otherwise
       static_for<0, Q7>([&](auto KK) {
@@ -929,14 +862,9 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
       st_at(s.rho[nxt], i, nCell, 18, rhoN);
       st_at(s.phi[nxt], i, nCell, 18, p);
       if constexpr (UPAD) {
-        // f's last group with ux in its pad (where SOLID links were written,
-        // the group went out above and only the pad remains)
-        if (orTags & TAG_SOLID) {
-          st_at(Fn, bF + pofs(27), nF, 18, (PopT)uxn);
-        } else {
-          lastF[3] = (PopT)uxn;
-          st4_at(Fn, bF + pofs(Q27 - 3), nF, 15, lastF);
-        }
+        // f's last group with ux in its pad
+        lastF[3] = (PopT)uxn;
+        st4_at(Fn, bF + pofs(Q27 - 3), nF, 15, lastF);
       } else {
         st_at(s.ux[nxt], i, nCell, 18, uxn);
         st_at(s.uy[nxt], i, nCell, 18, uyn);
@@ -952,7 +880,6 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
     gyC = gyN;
     gzC = gzN;
     lapC = lapN;
-    phC = phN;
   }
 
   // Stopped early (a wait ran out): the copy of stage q was issued (unless

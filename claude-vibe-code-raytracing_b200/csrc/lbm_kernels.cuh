@@ -368,43 +368,11 @@ __global__ void k_stream_hydro_macro(Scene<PopT, typename Prec<PopT>::Real> s, i
 // =====================================================================================
 // Sparse passes around the spheres.
 
-// retag on a box (the union of the current and the two previous sphere boxes):
-// every cell outside it keeps tag == tagPrev, so only the box changes.
-// (the bodies of the sparse kernels take their block index and grid size, so
-// that a batched launch can run them for many scenes, one grid row each)
-template <class PopT>
-__device__ __forceinline__ void retag_box_body(const Scene<PopT, typename Prec<PopT>::Real> &s,
-                                               const Plan *__restrict__ P, unsigned bid, unsigned gdim) {
-  const SolidSet &ss = P->ss;
-  const Box bx = P->U;
-  const int dx = bx.hi[0] - bx.lo[0] + 1, dy = bx.hi[1] - bx.lo[1] + 1, dz = bx.hi[2] - bx.lo[2] + 1;
-  const long long total = (long long)dx * dy * dz;
-  // grid-stride over the box the plan holds (launches are sized for the
-  // largest box the step may plan, which can be far larger)
-  for (long long l = bid * (long long)blockDim.x + threadIdx.x; l < total; l += (long long)gdim * blockDim.x) {
-    const int x = bx.lo[0] + (int)(l % dx);
-    const int y = bx.lo[1] + (int)((l / dx) % dy);
-    const int z = bx.lo[2] + (int)(l / ((long long)dx * dy));
-    const long long i = cell_index(x, y, z, s.nx, s.ny);
-    s.tagPrev[i] = s.tag[i];
-    if (x == 0 || x == s.nx - 1 || y == 0 || y == s.ny - 1 || z == 0 || z == s.nz - 1)
-      s.tag[i] = TAG_WALL;
-    else
-      s.tag[i] = owner_of<LBM_MAX_SPHERES>(ss.sph, ss.nsph, x, y, z) >= 0 ? TAG_SOLID : TAG_FLUID;
-  }
-}
-template <class PopT>
-__global__ void k_retag_box(Scene<PopT, typename Prec<PopT>::Real> s, const Plan *__restrict__ P) {
-  retag_box_body<PopT>(s, P, blockIdx.x, gridDim.x);
-}
-
-// Count fresh (FLUID, was SOLID) and dead (SOLID, was FLUID) cells per chunk
-// of the box's linear (scan) order.
+// Cells of a box in its linear (scan) order are worked on in chunks.
 constexpr int COMPACT_CHUNK = 2048;
-constexpr int COMPACT_THREADS = 256;
-// Most CTAs a box sweep (retag, compaction) launches: the kernels stride over
-// the box or its chunks, so a step whose planned box is small does not pay
-// for the empty CTAs of a launch sized for the largest possible box.
+// Most CTAs a box sweep launches: the kernels stride over the box's chunks, so
+// a step whose planned box is small does not pay for the empty CTAs of a
+// launch sized for the largest possible box.
 constexpr unsigned SWEEP_CTAS = 148 * 4;
 
 __device__ __forceinline__ void box_cell(const Box &bx, long long l, int &x, int &y, int &z) {
@@ -412,160 +380,6 @@ __device__ __forceinline__ void box_cell(const Box &bx, long long l, int &x, int
   x = bx.lo[0] + (int)(l % dx);
   y = bx.lo[1] + (int)((l / dx) % dy);
   z = bx.lo[2] + (int)(l / ((long long)dx * dy));
-}
-
-__device__ __forceinline__ void compact_count_body(const uint8_t *tag, const uint8_t *tagPrev, int nx, int ny,
-                                                   const Plan *__restrict__ P, int2 *counts, unsigned bid,
-                                                   unsigned gdim) {
-  __shared__ int sf[COMPACT_THREADS / 32], sd[COMPACT_THREADS / 32];
-  const Box bx = P->U;
-  const long long total = P->ucells;
-  const int nchunks = P->nchunks;
-  // CTAs stride over the chunks (block-uniform trip count)
-  for (int c = bid; c < nchunks; c += gdim) {
-    const long long base = (long long)c * COMPACT_CHUNK;
-    int nf = 0, nd = 0;
-    for (int j = threadIdx.x; j < COMPACT_CHUNK; j += blockDim.x) {
-      long long l = base + j;
-      if (l >= total) break;
-      int x, y, z;
-      box_cell(bx, l, x, y, z);
-      long long i = cell_index(x, y, z, nx, ny);
-      uint8_t t = tag[i], p = tagPrev[i];
-      nf += (t == TAG_FLUID && p == TAG_SOLID);
-      nd += (t == TAG_SOLID && p == TAG_FLUID);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      nf += __shfl_xor_sync(0xffffffffu, nf, o);
-      nd += __shfl_xor_sync(0xffffffffu, nd, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-      sf[threadIdx.x >> 5] = nf;
-      sd[threadIdx.x >> 5] = nd;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int a = 0, b = 0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
-        a += sf[w];
-        b += sd[w];
-      }
-      counts[c] = make_int2(a, b);
-    }
-    __syncthreads();  // sf / sd are rewritten for the next chunk
-  }
-}
-static __global__ void k_compact_count(const uint8_t *tag, const uint8_t *tagPrev, int nx, int ny,
-                                       const Plan *__restrict__ P, int2 *counts) {
-  compact_count_body(tag, tagPrev, nx, ny, P, counts, blockIdx.x, gridDim.x);
-}
-
-// Exclusive scan of the per-chunk counts (single CTA, sequential per thread).
-__device__ __forceinline__ void compact_scan_body(int2 *counts, const Plan *__restrict__ P, int *totals) {
-  __shared__ int2 part[1024];
-  const int nchunks = P->nchunks;
-  int per = (nchunks + blockDim.x - 1) / blockDim.x;
-  int b0 = threadIdx.x * per, b1 = min(b0 + per, nchunks);
-  int2 sum = make_int2(0, 0);
-  for (int b = b0; b < b1; b++) {
-    sum.x += counts[b].x;
-    sum.y += counts[b].y;
-  }
-  part[threadIdx.x] = sum;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int2 run = make_int2(0, 0);
-    for (int t = 0; t < (int)blockDim.x; t++) {
-      int2 v = part[t];
-      part[t] = run;
-      run.x += v.x;
-      run.y += v.y;
-    }
-    totals[0] = run.x;
-    totals[1] = run.y;
-  }
-  __syncthreads();
-  int2 run = part[threadIdx.x];
-  for (int b = b0; b < b1; b++) {
-    int2 v = counts[b];
-    counts[b] = run;
-    run.x += v.x;
-    run.y += v.y;
-  }
-}
-static __global__ void k_compact_scan(int2 *counts, const Plan *__restrict__ P, int *totals) {
-  compact_scan_body(counts, P, totals);
-}
-
-// Emit the fresh / dead cell indices in scan order.
-__device__ __forceinline__ void compact_emit_body(const uint8_t *tag, const uint8_t *tagPrev, int nx, int ny,
-                                                  const Plan *__restrict__ P, const int2 *offsets, int *fresh,
-                                                  int *dead, int cap, unsigned bid, unsigned gdim) {
-  __shared__ int wf[COMPACT_THREADS / 32], wd[COMPACT_THREADS / 32];
-  __shared__ int runF, runD;
-  const Box bx = P->U;
-  const long long total = P->ucells;
-  const int nchunks = P->nchunks;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  // CTAs stride over the chunks (block-uniform trip count); the inner loop
-  // ends on a barrier, so runF / runD are free to be reset for the next chunk
-  for (int c = bid; c < nchunks; c += gdim) {
-    const long long base = (long long)c * COMPACT_CHUNK;
-    if (threadIdx.x == 0) {
-      runF = offsets[c].x;
-      runD = offsets[c].y;
-    }
-    __syncthreads();
-    for (int j0 = 0; j0 < COMPACT_CHUNK; j0 += blockDim.x) {
-      long long l = base + j0 + threadIdx.x;
-      bool isF = false, isD = false;
-      long long i = 0;
-      if (l < total && j0 + (int)threadIdx.x < COMPACT_CHUNK) {
-        int x, y, z;
-        box_cell(bx, l, x, y, z);
-        i = cell_index(x, y, z, nx, ny);
-        uint8_t t = tag[i], p = tagPrev[i];
-        isF = (t == TAG_FLUID && p == TAG_SOLID);
-        isD = (t == TAG_SOLID && p == TAG_FLUID);
-      }
-      unsigned bf = __ballot_sync(0xffffffffu, isF), bd = __ballot_sync(0xffffffffu, isD);
-      if (lane == 0) {
-        wf[warp] = __popc(bf);
-        wd[warp] = __popc(bd);
-      }
-      __syncthreads();
-      int offF = runF, offD = runD;
-      for (int w = 0; w < warp; w++) {
-        offF += wf[w];
-        offD += wd[w];
-      }
-      unsigned below = (1u << lane) - 1u;
-      if (isF) {
-        int pos = offF + __popc(bf & below);
-        if (pos < cap) fresh[pos] = (int)i;
-      }
-      if (isD) {
-        int pos = offD + __popc(bd & below);
-        if (pos < cap) dead[pos] = (int)i;
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        int a = 0, b = 0;
-        for (int w = 0; w < nw; w++) {
-          a += wf[w];
-          b += wd[w];
-        }
-        runF += a;
-        runD += b;
-      }
-      __syncthreads();
-    }
-  }
-}
-static __global__ void k_compact_emit(const uint8_t *tag, const uint8_t *tagPrev, int nx, int ny,
-                                      const Plan *__restrict__ P, const int2 *offsets, int *fresh,
-                                      int *dead, int cap) {
-  compact_emit_body(tag, tagPrev, nx, ny, P, offsets, fresh, dead, cap, blockIdx.x, gridDim.x);
 }
 
 // One fresh cell (src/sim.js:264-308): the FLUID neighbours' phi, rho and u
@@ -584,7 +398,8 @@ __device__ __forceinline__ void fill_cell(const Scene<PopT, typename Prec<PopT>:
       for (int dx = -1; dx <= 1; dx++) {
         if (!dx && !dy && !dz) continue;
         long long j = i + ((long long)dz * ny + dy) * nx + dx;
-        if (s.tag[j] == TAG_FLUID) {
+        // (from L2: other blocks of the same launch may have written the tag)
+        if (__ldcg(s.tag + j) == TAG_FLUID) {
           Real vp, vr, vx_, vy_, vz_;
           nb(j, vp, vr, vx_, vy_, vz_);
           psum += (double)vp;
@@ -640,11 +455,9 @@ constexpr int FILL_THREADS = 256;
 // thread in list order (also used for lists longer than FILL_PAR_MAX).
 template <class PopT>
 __device__ __forceinline__ void fresh_fill_body(const Scene<PopT, typename Prec<PopT>::Real> &s, int cur,
-                                                const int *fresh, const int *totals, int cap, double rhoL,
-                                                double rhoG, int zlo, int zend, int sequential) {
+                                                const int *fresh, int nf, double rhoL, double rhoG, int zlo,
+                                                int zend, int sequential) {
   using Real = typename Prec<PopT>::Real;
-  int nf = totals[0];
-  if (nf > cap) nf = cap;
   const long long nxny = (long long)s.nx * s.ny;
   auto skip = [&](long long i) -> bool {
     if (zend <= 0) return false;
@@ -730,12 +543,192 @@ __device__ __forceinline__ void fresh_fill_body(const Scene<PopT, typename Prec<
     if (!__syncthreads_or(waiting)) break;
   }
 }
+// ---------------------------------------------------------------- retag, fresh / dead sets, fresh fill
+// Arguments of a scene's sparse kernels (by value for one scene; a batch reads
+// one block per scene from device memory).
 template <class PopT>
-__global__ void __launch_bounds__(FILL_THREADS)
-    k_fresh_fill(Scene<PopT, typename Prec<PopT>::Real> s, int cur, const int *fresh, const int *totals, int cap,
-                 double rhoL, double rhoG, int zlo, int zend, int sequential) {
-  if (blockIdx.x != 0) return;
-  fresh_fill_body<PopT>(s, cur, fresh, totals, cap, rhoL, rhoG, zlo, zend, sequential);
+struct SmallArgs {
+  Scene<PopT, typename Prec<PopT>::Real> s;
+  int cur, listCap, zlo, zend, seqFill;
+  const Plan *plan;
+  int2 *counts;     // per chunk of the box: fresh, dead cells; then their offsets
+  uint32_t *bits;   // per chunk: [64] pairs of fresh / dead ballot words
+  unsigned *ticket;
+  int *fresh, *dead, *totals;
+  double rhoL, rhoG;
+};
+
+// The first three parts of a step around the spheres in one launch: retagCells
+// on the plan's box (RETAG; src/sim.js:214-244: every cell outside the union of
+// the current and the two previous sphere boxes keeps tag == tagPrev), the
+// scan-ordered lists of fresh (FLUID, was SOLID) and dead (SOLID, was FLUID)
+// cells, and handleFreshCells (FILL).
+//
+// Blocks stride over the box's 2,048-cell chunks and leave one fresh and one
+// dead ballot word per 32 cells and the chunk's counts; the block that takes
+// the last ticket scans the counts, writes the lists in scan order from the
+// ballots, one warp per chunk, and fills the fresh cells.
+// Latency-bound: the boxes hold 10^3 to 10^5 cells, so what counts is the
+// number of dependent launches.  This one launch takes the place of five
+// (retag, count, scan, emit, fill).
+constexpr int SETS_THREADS = 256;
+constexpr int SETS_WORDS = COMPACT_CHUNK / 32;
+
+template <class PopT, bool RETAG, bool FILL>
+__device__ __forceinline__ void sets_body(const SmallArgs<PopT> &a, unsigned bid, unsigned gdim) {
+  using Real = typename Prec<PopT>::Real;
+  static_assert(SETS_THREADS == 256 && COMPACT_CHUNK == 2048, "eight cells per thread and chunk");
+  __shared__ int2 sw[SETS_THREADS / 32];
+  __shared__ bool last;
+  const Scene<PopT, Real> &s = a.s;
+  const SolidSet &ss = a.plan->ss;
+  const Box bx = a.plan->U;
+  const unsigned total = (unsigned)a.plan->ucells;
+  const int nch = a.plan->nchunks;
+  const unsigned nb = min(gdim, (unsigned)max(nch, 1));
+  if (bid >= nb) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned dx = bx.hi[0] - bx.lo[0] + 1, dy = bx.hi[1] - bx.lo[1] + 1;
+  for (int c = bid; c < nch; c += gdim) {
+    int cell[8];
+    int3 at[8];
+    uint8_t t[8], p[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const unsigned l = (unsigned)c * COMPACT_CHUNK + j * SETS_THREADS + threadIdx.x;
+      cell[j] = -1;
+      if (l < total) {
+        const unsigned q = l / dx;
+        const int x = bx.lo[0] + (int)(l - q * dx), y = bx.lo[1] + (int)(q % dy), z = bx.lo[2] + (int)(q / dy);
+        cell[j] = (z * s.ny + y) * s.nx + x;
+        at[j] = make_int3(x, y, z);
+        t[j] = s.tag[cell[j]];
+        if (!RETAG) p[j] = s.tagPrev[cell[j]];
+      }
+    }
+    int nf = 0, nd = 0;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      bool isF = false, isD = false;
+      if (cell[j] >= 0) {
+        if (RETAG) {
+          const int x = at[j].x, y = at[j].y, z = at[j].z;
+          p[j] = t[j];
+          if (x == 0 || x == s.nx - 1 || y == 0 || y == s.ny - 1 || z == 0 || z == s.nz - 1) {
+            t[j] = TAG_WALL;
+          } else {
+            t[j] = owner_of<LBM_MAX_SPHERES>(ss.sph, ss.nsph, x, y, z) >= 0 ? TAG_SOLID : TAG_FLUID;
+          }
+          s.tagPrev[cell[j]] = p[j];
+          s.tag[cell[j]] = t[j];
+        }
+        isF = t[j] == TAG_FLUID && p[j] == TAG_SOLID;
+        isD = t[j] == TAG_SOLID && p[j] == TAG_FLUID;
+      }
+      const unsigned bf = __ballot_sync(0xffffffffu, isF), bd = __ballot_sync(0xffffffffu, isD);
+      if (lane == 0)
+        reinterpret_cast<uint2 *>(a.bits)[(long long)c * SETS_WORDS + j * (SETS_THREADS / 32) + warp] =
+            make_uint2(bf, bd);
+      nf += __popc(bf);
+      nd += __popc(bd);
+    }
+    if (lane == 0) sw[warp] = make_int2(nf, nd);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int2 v = make_int2(0, 0);
+      for (int w = 0; w < SETS_THREADS / 32; w++) v.x += sw[w].x, v.y += sw[w].y;
+      a.counts[c] = v;
+    }
+    __syncthreads();
+  }
+  if (nb > 1) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(a.ticket, 1u) == nb - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (threadIdx.x == 0) *a.ticket = 0;
+  }
+
+  // exclusive scan of the counts: each thread a run of chunks, then the block
+  const int per = (nch + SETS_THREADS - 1) / SETS_THREADS;
+  const int b0 = threadIdx.x * per, b1 = min(b0 + per, nch);
+  int2 sum = make_int2(0, 0);
+  for (int b = b0; b < b1; b++) {
+    const int2 v = __ldcg(a.counts + b);
+    sum.x += v.x;
+    sum.y += v.y;
+  }
+  int2 inc = sum;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int fx = __shfl_up_sync(0xffffffffu, inc.x, o), fy = __shfl_up_sync(0xffffffffu, inc.y, o);
+    if (lane >= o) inc.x += fx, inc.y += fy;
+  }
+  if (lane == 31) sw[warp] = inc;
+  __syncthreads();
+  int2 run = make_int2(inc.x - sum.x, inc.y - sum.y), all = make_int2(0, 0);
+  for (int w = 0; w < SETS_THREADS / 32; w++) {
+    if (w < warp) run.x += sw[w].x, run.y += sw[w].y;
+    all.x += sw[w].x, all.y += sw[w].y;
+  }
+  if (threadIdx.x == 0) {
+    a.totals[0] = all.x;
+    a.totals[1] = all.y;
+  }
+  if (all.x == 0 && all.y == 0) return;
+  // offsets of the chunks that hold any (y < 0 marks the others)
+  for (int b = b0; b < b1; b++) {
+    const int2 v = __ldcg(a.counts + b);
+    a.counts[b] = v.x | v.y ? run : make_int2(0, -1);
+    run.x += v.x;
+    run.y += v.y;
+  }
+  __syncthreads();
+  // one warp per such chunk: lane l's two words of 32 cells each, in order
+  for (int c0 = warp * 32; c0 < nch; c0 += SETS_THREADS) {
+    const int2 off = c0 + lane < nch ? a.counts[c0 + lane] : make_int2(0, -1);
+    unsigned busy = __ballot_sync(0xffffffffu, off.y >= 0);
+    for (; busy; busy &= busy - 1) {
+      const int src = __ffs(busy) - 1, c = c0 + src;
+      int of = __shfl_sync(0xffffffffu, off.x, src), od = __shfl_sync(0xffffffffu, off.y, src);
+      const uint4 w = __ldcg(reinterpret_cast<const uint4 *>(a.bits) + (long long)c * (SETS_WORDS / 2) + lane);
+      const int mf = __popc(w.x) + __popc(w.z), md = __popc(w.y) + __popc(w.w);
+      int pf = mf, pd = md;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, pf, o), y = __shfl_up_sync(0xffffffffu, pd, o);
+        if (lane >= o) pf += x, pd += y;
+      }
+      of += pf - mf;
+      od += pd - md;
+      for (int h = 0; h < 2; h++) {
+        const unsigned l0 = (unsigned)c * COMPACT_CHUNK + (2 * lane + h) * 32;
+        auto put = [&](unsigned m, int *list, int &pos) {
+          for (; m; m &= m - 1, pos++) {
+            int x, y, z;
+            box_cell(bx, l0 + (__ffs(m) - 1), x, y, z);
+            if (pos < a.listCap) list[pos] = (z * s.ny + y) * s.nx + x;
+          }
+        };
+        put(h ? w.z : w.x, a.fresh, of);
+        put(h ? w.w : w.y, a.dead, od);
+      }
+    }
+  }
+  if constexpr (FILL) {
+    if (all.x == 0) return;
+    __syncthreads();
+    fresh_fill_body<PopT>(s, a.cur, a.fresh, min(all.x, a.listCap), a.rhoL, a.rhoG, a.zlo, a.zend, a.seqFill);
+  }
+}
+template <class PopT, bool RETAG, bool FILL>
+__global__ void __launch_bounds__(SETS_THREADS) k_sets(const __grid_constant__ SmallArgs<PopT> a) {
+  sets_body<PopT, RETAG, FILL>(a, blockIdx.x, gridDim.x);
+}
+// every scene of a batch: grid row s is scene s
+template <class PopT>
+__global__ void __launch_bounds__(SETS_THREADS) kb_sets(const SmallArgs<PopT> *__restrict__ A) {
+  sets_body<PopT, true, true>(A[blockIdx.y], blockIdx.x, gridDim.x);
 }
 
 // absorbDeadCells (src/solid.js:87-101): impulse rho(phi)*u of every cell on
@@ -895,12 +888,15 @@ template <class Fields>
 __device__ __forceinline__ void absorb_dead_body(const Fields &fd, int nx, int ny, const int *__restrict__ dead,
                                                  const int *__restrict__ totals, int cap, double rhoL,
                                                  double rhoG, const SolidSet *__restrict__ ssp, double *out,
-                                                 int b) {
-  __shared__ double sh[6][DEAD_THREADS];
+                                                 int b, double (*sh)[DEAD_THREADS]) {
   const SolidSet &ss = *ssp;
   if (b >= ss.nsph) return;
   int nd = totals[1];
   if (nd > cap) nd = cap;
+  if (nd == 0) {
+    if (threadIdx.x < 6) out[6 * b + threadIdx.x] = 0.0;
+    return;
+  }
   const double dRho = rhoL - rhoG;
   const int per = (nd + DEAD_THREADS - 1) / DEAD_THREADS;
   const int q0 = threadIdx.x * per, q1 = min(q0 + per, nd);
@@ -925,6 +921,7 @@ __device__ __forceinline__ void absorb_dead_body(const Fields &fd, int nx, int n
     __syncthreads();
   }
   if (threadIdx.x < 6) out[6 * b + threadIdx.x] = sh[threadIdx.x][0];
+  __syncthreads();
 }
 template <class Real>
 static __global__ void __launch_bounds__(DEAD_THREADS)
@@ -932,8 +929,9 @@ static __global__ void __launch_bounds__(DEAD_THREADS)
                   const Real *__restrict__ uy, const Real *__restrict__ uz, int nx, int ny,
                   const int *__restrict__ dead, const int *__restrict__ totals, int cap, double rhoL,
                   double rhoG, const SolidSet *__restrict__ ssp, double *out) {
+  __shared__ double sh[6][DEAD_THREADS];
   absorb_dead_body(ArrayFields<Real>{phi, ux, uy, uz}, nx, ny, dead, totals, cap, rhoL, rhoG, ssp, out,
-                   blockIdx.x);
+                   blockIdx.x, sh);
 }
 // the same over a scene's current half
 template <class PopT>
@@ -941,7 +939,9 @@ static __global__ void __launch_bounds__(DEAD_THREADS)
     k_absorb_dead_scene(Scene<PopT, typename Prec<PopT>::Real> s, int cur, const int *__restrict__ dead,
                         const int *__restrict__ totals, int cap, double rhoL, double rhoG,
                         const SolidSet *__restrict__ ssp, double *out) {
-  absorb_dead_body(SceneFields<PopT>{s, cur}, s.nx, s.ny, dead, totals, cap, rhoL, rhoG, ssp, out, blockIdx.x);
+  __shared__ double sh[6][DEAD_THREADS];
+  absorb_dead_body(SceneFields<PopT>{s, cur}, s.nx, s.ny, dead, totals, cap, rhoL, rhoG, ssp, out, blockIdx.x,
+                   sh);
 }
 
 // Deterministic reduction of the per-cell impulse arrays in one launch.
@@ -1015,36 +1015,41 @@ static __global__ void __launch_bounds__(RED_THREADS)
   impulse_reduce_body(ssp, partials, maxChunks, out, tickets, blockIdx.x, blockIdx.y);
 }
 
-// Device-side plan for the device-resident loop: sphere descriptors from the
-// device sphere state, the retag box (current and two previous sphere boxes),
+// Device-side plan P of a step of the device-resident loop, from the sphere
+// state and the previous step's plan (the same object for the first step):
+// sphere descriptors, the retag box (current and two previous sphere boxes),
 // compaction chunking, and impulse slots of slotCells cells per sphere.
-__device__ __forceinline__ void plan_body(Plan *P, const lbm_sphere *sph, int nsph, int nx, int ny, int nz,
-                                          double *impBase, long long slotCells, long long maxUCells) {
-  if (threadIdx.x != 0) return;
+__device__ __forceinline__ void plan_body(Plan *P, const Plan *prev, const lbm_sphere *sph, int nsph, int nx, int ny,
+                                          int nz, double *impBase, long long slotCells, long long maxUCells) {
   SolidSet &ss = P->ss;
+  const Box boxLast = prev->boxLast, boxLastLast = prev->boxLastLast;
+  const int fullRetag = prev->fullRetag;
+  int overflow = prev->overflow;
   ss.nsph = nsph;
+  ss.zlo = ss.zend = 0;
   Box now{{1, 1, 1}, {0, 0, 0}};
   int redChunks = 1;
   for (int b = 0; b < nsph; b++) {
     SphereDesc &d = ss.sph[b];
-    d.cx = sph[b].cx;
-    d.cy = sph[b].cy;
-    d.cz = sph[b].cz;
-    d.r = sph[b].r;
+    const double cx = sph[b].cx, cy = sph[b].cy, cz = sph[b].cz, r = sph[b].r;
+    d.cx = cx;
+    d.cy = cy;
+    d.cz = cz;
+    d.r = r;
     d.vx = sph[b].vx;
     d.vy = sph[b].vy;
     d.vz = sph[b].vz;
     d.wx = sph[b].wx;
     d.wy = sph[b].wy;
     d.wz = sph[b].wz;
-    Box sb = sphere_box(d.cx, d.cy, d.cz, d.r, nx, ny, nz);
+    const Box sb = sphere_box(cx, cy, cz, r, nx, ny, nz);
     now = box_union(now, sb);
     Box tb = box_grow(sb, 1, nx, ny, nz);
     ImpulseTarget &t = ss.imp[b];
     t.acc = impBase + (long long)b * slotCells * 6;
     long long cells = box_cells(tb);
     if (cells > slotCells) {
-      P->overflow = 1;
+      overflow = 1;
       cells = 0;
       tb = Box{{1, 1, 1}, {0, 0, 0}};
     }
@@ -1052,34 +1057,36 @@ __device__ __forceinline__ void plan_body(Plan *P, const lbm_sphere *sph, int ns
       t.lo[a] = box_empty(tb) ? 0 : tb.lo[a];
       t.dim[a] = box_empty(tb) ? 0 : tb.hi[a] - tb.lo[a] + 1;
     }
-    int rc = (int)((cells + RED_CHUNK - 1) / RED_CHUNK);
+    const int rc = (int)((cells + RED_CHUNK - 1) / RED_CHUNK);
     redChunks = rc > redChunks ? rc : redChunks;
   }
   Box U;
-  if (P->fullRetag > 0) {
+  if (fullRetag > 0) {
     U = Box{{0, 0, 0}, {nx - 1, ny - 1, nz - 1}};
-    P->fullRetag--;
+    P->fullRetag = fullRetag - 1;
   } else {
-    U = box_union(box_union(now, P->boxLast), P->boxLastLast);
+    U = box_union(box_union(now, boxLast), boxLastLast);
+    P->fullRetag = 0;
   }
   long long uc = box_cells(U);
   if (uc > maxUCells) {
-    P->overflow = 1;
+    overflow = 1;
     uc = 0;
     U = Box{{1, 1, 1}, {0, 0, 0}};
   }
+  P->overflow = overflow;
   P->U = U;
   P->ucells = uc;
   P->nchunks = (int)((uc + COMPACT_CHUNK - 1) / COMPACT_CHUNK);
   P->redChunks = redChunks;
   P->impDoubles = (long long)nsph * slotCells * 6;
-  P->boxLastLast = P->boxLast;
+  P->boxLastLast = boxLast;
   P->boxLast = now;
 }
-static __global__ void k_plan(Plan *P, const lbm_sphere *sph, int nsph, int nx, int ny, int nz,
-                              double *impBase, long long slotCells, long long maxUCells) {
-  if (blockIdx.x != 0) return;
-  plan_body(P, sph, nsph, nx, ny, nz, impBase, slotCells, maxUCells);
+static __global__ void k_plan(Plan *P, const lbm_sphere *sph, int nsph, int nx, int ny, int nz, double *impBase,
+                              long long slotCells, long long maxUCells) {
+  if (blockIdx.x == 0 && threadIdx.x == 0)
+    plan_body(P, P, sph, nsph, nx, ny, nz, impBase, slotCells, maxUCells);
 }
 
 // packVolume's two bytes of cell i (src/sim.js:586-600): R = clamp01(phi) *

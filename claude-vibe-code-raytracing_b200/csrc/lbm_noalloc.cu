@@ -38,6 +38,164 @@ using namespace lbm;
 
 namespace {
 
+constexpr int COMPACT_THREADS = 256;
+
+// Count fresh (FLUID, was SOLID) and dead (SOLID, was FLUID) cells per chunk
+// of the box's linear (scan) order.
+__device__ __forceinline__ void compact_count_body(const uint8_t *tag, const uint8_t *tagPrev, int nx, int ny,
+                                                   const Plan *__restrict__ P, int2 *counts, unsigned bid,
+                                                   unsigned gdim) {
+  __shared__ int sf[COMPACT_THREADS / 32], sd[COMPACT_THREADS / 32];
+  const Box bx = P->U;
+  const long long total = P->ucells;
+  const int nchunks = P->nchunks;
+  // CTAs stride over the chunks (block-uniform trip count)
+  for (int c = bid; c < nchunks; c += gdim) {
+    const long long base = (long long)c * COMPACT_CHUNK;
+    int nf = 0, nd = 0;
+    for (int j = threadIdx.x; j < COMPACT_CHUNK; j += blockDim.x) {
+      long long l = base + j;
+      if (l >= total) break;
+      int x, y, z;
+      box_cell(bx, l, x, y, z);
+      long long i = cell_index(x, y, z, nx, ny);
+      uint8_t t = tag[i], p = tagPrev[i];
+      nf += (t == TAG_FLUID && p == TAG_SOLID);
+      nd += (t == TAG_SOLID && p == TAG_FLUID);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      nf += __shfl_xor_sync(0xffffffffu, nf, o);
+      nd += __shfl_xor_sync(0xffffffffu, nd, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+      sf[threadIdx.x >> 5] = nf;
+      sd[threadIdx.x >> 5] = nd;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int a = 0, b = 0;
+      for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
+        a += sf[w];
+        b += sd[w];
+      }
+      counts[c] = make_int2(a, b);
+    }
+    __syncthreads();  // sf / sd are rewritten for the next chunk
+  }
+}
+__global__ void k_compact_count(const uint8_t *tag, const uint8_t *tagPrev, int nx, int ny,
+                                       const Plan *__restrict__ P, int2 *counts) {
+  compact_count_body(tag, tagPrev, nx, ny, P, counts, blockIdx.x, gridDim.x);
+}
+
+// Exclusive scan of the per-chunk counts (single CTA, sequential per thread).
+__device__ __forceinline__ void compact_scan_body(int2 *counts, const Plan *__restrict__ P, int *totals) {
+  __shared__ int2 part[1024];
+  const int nchunks = P->nchunks;
+  int per = (nchunks + blockDim.x - 1) / blockDim.x;
+  int b0 = threadIdx.x * per, b1 = min(b0 + per, nchunks);
+  int2 sum = make_int2(0, 0);
+  for (int b = b0; b < b1; b++) {
+    sum.x += counts[b].x;
+    sum.y += counts[b].y;
+  }
+  part[threadIdx.x] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int2 run = make_int2(0, 0);
+    for (int t = 0; t < (int)blockDim.x; t++) {
+      int2 v = part[t];
+      part[t] = run;
+      run.x += v.x;
+      run.y += v.y;
+    }
+    totals[0] = run.x;
+    totals[1] = run.y;
+  }
+  __syncthreads();
+  int2 run = part[threadIdx.x];
+  for (int b = b0; b < b1; b++) {
+    int2 v = counts[b];
+    counts[b] = run;
+    run.x += v.x;
+    run.y += v.y;
+  }
+}
+__global__ void k_compact_scan(int2 *counts, const Plan *__restrict__ P, int *totals) {
+  compact_scan_body(counts, P, totals);
+}
+
+// Emit the fresh / dead cell indices in scan order.
+__device__ __forceinline__ void compact_emit_body(const uint8_t *tag, const uint8_t *tagPrev, int nx, int ny,
+                                                  const Plan *__restrict__ P, const int2 *offsets, int *fresh,
+                                                  int *dead, int cap, unsigned bid, unsigned gdim) {
+  __shared__ int wf[COMPACT_THREADS / 32], wd[COMPACT_THREADS / 32];
+  __shared__ int runF, runD;
+  const Box bx = P->U;
+  const long long total = P->ucells;
+  const int nchunks = P->nchunks;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  // CTAs stride over the chunks (block-uniform trip count); the inner loop
+  // ends on a barrier, so runF / runD are free to be reset for the next chunk
+  for (int c = bid; c < nchunks; c += gdim) {
+    const long long base = (long long)c * COMPACT_CHUNK;
+    if (threadIdx.x == 0) {
+      runF = offsets[c].x;
+      runD = offsets[c].y;
+    }
+    __syncthreads();
+    for (int j0 = 0; j0 < COMPACT_CHUNK; j0 += blockDim.x) {
+      long long l = base + j0 + threadIdx.x;
+      bool isF = false, isD = false;
+      long long i = 0;
+      if (l < total && j0 + (int)threadIdx.x < COMPACT_CHUNK) {
+        int x, y, z;
+        box_cell(bx, l, x, y, z);
+        i = cell_index(x, y, z, nx, ny);
+        uint8_t t = tag[i], p = tagPrev[i];
+        isF = (t == TAG_FLUID && p == TAG_SOLID);
+        isD = (t == TAG_SOLID && p == TAG_FLUID);
+      }
+      unsigned bf = __ballot_sync(0xffffffffu, isF), bd = __ballot_sync(0xffffffffu, isD);
+      if (lane == 0) {
+        wf[warp] = __popc(bf);
+        wd[warp] = __popc(bd);
+      }
+      __syncthreads();
+      int offF = runF, offD = runD;
+      for (int w = 0; w < warp; w++) {
+        offF += wf[w];
+        offD += wd[w];
+      }
+      unsigned below = (1u << lane) - 1u;
+      if (isF) {
+        int pos = offF + __popc(bf & below);
+        if (pos < cap) fresh[pos] = (int)i;
+      }
+      if (isD) {
+        int pos = offD + __popc(bd & below);
+        if (pos < cap) dead[pos] = (int)i;
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        int a = 0, b = 0;
+        for (int w = 0; w < nw; w++) {
+          a += wf[w];
+          b += wd[w];
+        }
+        runF += a;
+        runD += b;
+      }
+      __syncthreads();
+    }
+  }
+}
+__global__ void k_compact_emit(const uint8_t *tag, const uint8_t *tagPrev, int nx, int ny,
+                                      const Plan *__restrict__ P, const int2 *offsets, int *fresh,
+                                      int *dead, int cap) {
+  compact_emit_body(tag, tagPrev, nx, ny, P, offsets, fresh, dead, cap, blockIdx.x, gridDim.x);
+}
+
 constexpr long long NOALLOC_MAX_BOX = 1LL << 20;  // cells of the search box
 constexpr int NOALLOC_MAX_CHUNKS = (int)(NOALLOC_MAX_BOX / COMPACT_CHUNK);
 constexpr int NOALLOC_MAX_DEVICES = 64;

@@ -9,6 +9,7 @@
 
 #include "lbm_fused_pipe.cuh"
 #include "lbm_kernels.cuh"
+#include "lbm_shell.cuh"
 #include "lbm_sphere.cuh"
 #include "lbm_state.h"
 
@@ -85,34 +86,6 @@ __global__ void k_reencode_h(Scene<PopT, typename Prec<PopT>::Real> s, int half,
   }
 }
 
-// The device-resident loop's RigidSphere.step(1.0, gravity), one thread per
-// sphere: the momentum-exchange and dead-cell impulses of the step are added
-// first, as RigidSphere.applyImpulseAtCell would have.
-__device__ __forceinline__ void sphere_step_body(lbm_sphere *sph, int nsph, double gravity, const double *fluid,
-                                                 const double *dead, int nx, int ny, int nz) {
-  int b = threadIdx.x;
-  if (b >= nsph) return;
-  lbm_sphere s = sph[b];
-  double *F[6] = {&s.Fx, &s.Fy, &s.Fz, &s.Tx, &s.Ty, &s.Tz};
-  for (int j = 0; j < 6; j++) {
-    if (fluid) *F[j] = __dadd_rn(*F[j], fluid[6 * b + j]);
-    if (dead) *F[j] = __dadd_rn(*F[j], dead[6 * b + j]);
-  }
-  sphere_step_fp64(s, 1.0, gravity, nx, ny, nz);
-  sph[b] = s;
-}
-static __global__ void k_sphere_step(lbm_sphere *sph, int nsph, double gravity, const double *fluid,
-                                     const double *dead, int nx, int ny, int nz) {
-  if (blockIdx.x != 0) return;
-  sphere_step_body(sph, nsph, gravity, fluid, dead, nx, ny, nz);
-}
-
-// ---------------------------------------------------------------- batched sparse kernels
-// A batch runs every scene's sparse kernels of a step (plan, retag, fresh /
-// dead compaction, fresh fill; after the shared fused launch the impulse
-// reduction, the dead-cell impulses and the sphere step) as one launch per
-// kind: grid row (or plane) s runs scene s's kernel body on scene s's
-// arguments, so a step of n scenes costs 9 launches instead of 9 n.
 // ux (comp 0) or uy (comp 1) of one half between a plain array and the
 // place the scene keeps it (Scene::ux_at / set_ux), for the field transfers
 template <class PopT>
@@ -126,72 +99,6 @@ __global__ void k_u_array(Scene<PopT, typename Prec<PopT>::Real> s, int comp, in
   } else {
     arr[i] = comp == 0 ? s.ux_at(half, i) : s.uy_at(half, i);
   }
-}
-
-template <class PopT>
-struct SmallArgs {
-  Scene<PopT, typename Prec<PopT>::Real> s;
-  int cur, ns, listCap, redChunks, zlo, zend, seqFill;
-  Plan *plan;
-  lbm_sphere *sph;
-  double *impAcc;
-  long long slotCells, maxU;
-  int2 *counts;
-  int *fresh, *dead, *totals;
-  double *partials, *dFluid, *dDead;
-  unsigned *tickets;
-  double rhoL, rhoG, gravity;
-};
-
-template <class PopT>
-__global__ void kb_plan(const SmallArgs<PopT> *__restrict__ A) {
-  const SmallArgs<PopT> &a = A[blockIdx.x];
-  plan_body(a.plan, a.sph, a.ns, a.s.nx, a.s.ny, a.s.nz, a.impAcc, a.slotCells, a.maxU);
-}
-template <class PopT>
-__global__ void kb_retag_box(const SmallArgs<PopT> *__restrict__ A) {
-  const SmallArgs<PopT> &a = A[blockIdx.y];
-  retag_box_body<PopT>(a.s, a.plan, blockIdx.x, gridDim.x);
-}
-template <class PopT>
-__global__ void kb_compact_count(const SmallArgs<PopT> *__restrict__ A) {
-  const SmallArgs<PopT> &a = A[blockIdx.y];
-  compact_count_body(a.s.tag, a.s.tagPrev, a.s.nx, a.s.ny, a.plan, a.counts, blockIdx.x, gridDim.x);
-}
-template <class PopT>
-__global__ void kb_compact_scan(const SmallArgs<PopT> *__restrict__ A) {
-  const SmallArgs<PopT> &a = A[blockIdx.x];
-  compact_scan_body(a.counts, a.plan, a.totals);
-}
-template <class PopT>
-__global__ void kb_compact_emit(const SmallArgs<PopT> *__restrict__ A) {
-  const SmallArgs<PopT> &a = A[blockIdx.y];
-  compact_emit_body(a.s.tag, a.s.tagPrev, a.s.nx, a.s.ny, a.plan, a.counts, a.fresh, a.dead, a.listCap,
-                    blockIdx.x, gridDim.x);
-}
-template <class PopT>
-__global__ void __launch_bounds__(FILL_THREADS) kb_fresh_fill(const SmallArgs<PopT> *__restrict__ A) {
-  const SmallArgs<PopT> &a = A[blockIdx.x];
-  fresh_fill_body<PopT>(a.s, a.cur, a.fresh, a.totals, a.listCap, a.rhoL, a.rhoG, a.zlo, a.zend, a.seqFill);
-}
-template <class PopT>
-__global__ void __launch_bounds__(RED_THREADS) kb_impulse_reduce(const SmallArgs<PopT> *__restrict__ A) {
-  const SmallArgs<PopT> &a = A[blockIdx.z];
-  if (a.ns == 0) return;
-  impulse_reduce_body(&a.plan->ss, a.partials, a.redChunks, a.dFluid, a.tickets, blockIdx.x, blockIdx.y);
-}
-template <class PopT>
-__global__ void __launch_bounds__(DEAD_THREADS) kb_absorb_dead(const SmallArgs<PopT> *__restrict__ A) {
-  const SmallArgs<PopT> &a = A[blockIdx.y];
-  if (a.ns == 0) return;
-  absorb_dead_body(SceneFields<PopT>{a.s, a.cur}, a.s.nx, a.s.ny, a.dead, a.totals, a.listCap, a.rhoL, a.rhoG,
-                   &a.plan->ss, a.dDead, blockIdx.x);
-}
-template <class PopT>
-__global__ void kb_sphere_step(const SmallArgs<PopT> *__restrict__ A) {
-  const SmallArgs<PopT> &a = A[blockIdx.x];
-  if (a.ns == 0) return;
-  sphere_step_body(a.sph, a.ns, a.gravity, a.dFluid, a.dDead, a.s.nx, a.s.ny, a.s.nz);
 }
 
 // ---------------------------------------------------------------- launcher
@@ -252,7 +159,7 @@ class Ops final : public OpsBase {
     h->launches++;
   }
   void retag_full(lbm_sim *h) override {
-    k_retag_full<PopT><<<nblocks(h->n, 256), 256, 0, h->stream>>>(scene(h), h->cur, &h->dPlan->ss);
+    k_retag_full<PopT><<<nblocks(h->n, 256), 256, 0, h->stream>>>(scene(h), h->cur, &h->plan()->ss);
     h->launches++;
   }
   void retag_mask(lbm_sim *h, const uint8_t *d_mask, const float *d_us) override {
@@ -286,26 +193,42 @@ class Ops final : public OpsBase {
   }
   void stream_hydro_macro(lbm_sim *h) override {
     k_stream_hydro_macro<PopT><<<nblocks(h->n, 256), 256, 0, h->stream>>>(
-        scene(h), h->cur, make_const(h->params), &h->dPlan->ss);
+        scene(h), h->cur, make_const(h->params), &h->plan()->ss);
     h->launches++;
   }
-  void retag_box(lbm_sim *h, long long maxCells) override {
-    if (maxCells <= 0) return;
-    k_retag_box<PopT><<<std::min(nblocks(maxCells, 256), SWEEP_CTAS), 256, 0, h->stream>>>(scene(h), h->dPlan);
-    h->launches++;
+  // the sparse kernels' arguments for the step that reads half cur
+  static SmallArgs<PopT> small(lbm_sim *h, int cur) {
+    SmallArgs<PopT> a;
+    a.s = scene(h);
+    a.cur = cur;
+    a.listCap = (int)h->listCap;
+    a.zlo = h->slab ? h->ownLo : 0;
+    a.zend = h->slab ? h->ownHi + 1 : 0;
+    a.seqFill = h->sequentialFill ? 1 : 0;
+    a.plan = h->dPlan + cur;
+    a.counts = h->counts;
+    a.bits = (uint32_t *)h->setBits;
+    a.ticket = h->redTickets + LBM_MAX_SPHERES;
+    a.fresh = h->fresh;
+    a.dead = h->dead;
+    a.totals = h->totals;
+    a.rhoL = h->params.rhoL;
+    a.rhoG = h->params.rhoG;
+    return a;
   }
-  void fresh_fill(lbm_sim *h) override {
-    k_fresh_fill<PopT><<<1, FILL_THREADS, 0, h->stream>>>(scene(h), h->cur, h->fresh, h->totals,
-                                                           (int)h->listCap, h->params.rhoL, h->params.rhoG,
-                                                           h->slab ? h->ownLo : 0, h->slab ? h->ownHi + 1 : 0,
-                                                           h->sequentialFill ? 1 : 0);
+  void sets(lbm_sim *h, long long maxChunks, bool retag, bool fill) override {
+    const unsigned ctas = (unsigned)std::min<long long>(std::max(1LL, maxChunks), SWEEP_CTAS);
+    const SmallArgs<PopT> a = small(h, h->cur);
+    if (retag) k_sets<PopT, true, true><<<ctas, SETS_THREADS, 0, h->stream>>>(a);
+    else if (fill) k_sets<PopT, false, true><<<ctas, SETS_THREADS, 0, h->stream>>>(a);
+    else k_sets<PopT, false, false><<<ctas, SETS_THREADS, 0, h->stream>>>(a);
     h->launches++;
   }
   void absorb_dead(lbm_sim *h, double *d_out) override {
     const int ns = h->hPlan.ss.nsph > 0 ? h->hPlan.ss.nsph : 1;
     k_absorb_dead_scene<PopT><<<ns, DEAD_THREADS, 0, h->stream>>>(scene(h), h->cur, h->dead, h->totals,
                                                                   (int)h->listCap, h->params.rhoL,
-                                                                  h->params.rhoG, &h->dPlan->ss, d_out);
+                                                                  h->params.rhoG, &h->plan()->ss, d_out);
     h->launches++;
   }
 
@@ -351,14 +274,14 @@ class Ops final : public OpsBase {
   }
   // shared memory, warps and kernels of a launch form
   template <int TY, int FORM>
-  static constexpr size_t smem_of() {
-    if constexpr (FORM == 0) return FusedSmem<PopT, TY>::bytes;
-    else return PipeSmem<PopT, TY, FORM>::bytes;
-  }
-  template <int TY, int FORM>
   static constexpr int warps_of() {
     if constexpr (FORM == 0) return FusedSmem<PopT, TY>::warps;
     else return PipeSmem<PopT, TY, FORM>::warps;
+  }
+  template <int TY, int FORM>
+  static constexpr size_t smem_of() {
+    if constexpr (FORM == 0) return FusedSmem<PopT, TY>::bytes;
+    else return PipeSmem<PopT, TY, FORM>::bytes;
   }
   template <int TY, int FORM, bool WIDE, bool PACK = false>
   static auto step_kernel() {
@@ -408,7 +331,6 @@ class Ops final : public OpsBase {
     a.dRho = k.dRho;
     a.gravity = k.gravity;
     a.sharpC4 = 4 * k.sharpC;
-    a.ss = &h->dPlan->ss;
     a.status = h->totals + 2;
     a.withhold = h->withholdStage ? 1 : 0;
     a.pack = h->fusePack;
@@ -419,6 +341,32 @@ class Ops final : public OpsBase {
   void fused_args(lbm_sim *h, int cur, int zchunk, void *out) override {
     FusedArgs<PopT> a = make_args(h, cur, zchunk);
     memcpy(out, &a, sizeof(a));
+  }
+  ShellArgs<PopT> make_shell(lbm_sim *h, const StepCtx &c, int cur) {
+    ShellArgs<PopT> a;
+    memset((void *)&a, 0, sizeof(a));
+    a.f = make_args(h, cur, 1);
+    a.plan = h->dPlan + cur;
+    a.rhoL = h->params.rhoL;
+    a.ns = c.ns;
+    a.redChunks = std::max(1, c.redChunks);
+    a.listCap = (int)h->listCap;
+    a.ticket = h->redTickets;
+    a.partials = h->partials;
+    a.impulse = h->dOut;
+    a.dead = h->dead;
+    a.totals = h->totals;
+    a.sph = c.tail ? h->dSph : nullptr;
+    a.next = c.tail ? h->dPlan + (1 - cur) : nullptr;
+    a.impBase = h->impAcc;
+    a.slotCells = c.slotCells;
+    a.maxU = c.maxU;
+    return a;
+  }
+  void shell(lbm_sim *h, const StepCtx &c) override {
+    k_shell<PopT><<<dim3(std::max(1, c.redChunks), std::max(1, c.ns)), SHELL_THREADS, 0, h->stream>>>(
+        make_shell(h, c, h->cur));
+    h->launches++;
   }
   template <int TY, int STG, bool WIDE>
   int batch_ctas(int device) {
@@ -491,51 +439,24 @@ class Ops final : public OpsBase {
     h->launches++;
   }
   size_t small_args_bytes() const override { return sizeof(SmallArgs<PopT>); }
-  void small_args(lbm_sim *h, int cur, int ns, long long slotCells, long long maxU, int redChunks,
-                  void *out) override {
-    SmallArgs<PopT> a;
-    memset(&a, 0, sizeof(a));
-    a.s = scene(h);
-    a.cur = cur;
-    a.ns = ns;
-    a.listCap = (int)h->listCap;
-    a.redChunks = redChunks;
-    a.zlo = h->slab ? h->ownLo : 0;
-    a.zend = h->slab ? h->ownHi + 1 : 0;
-    a.seqFill = h->sequentialFill ? 1 : 0;
-    a.plan = h->dPlan;
-    a.sph = h->dSph;
-    a.impAcc = h->impAcc;
-    a.slotCells = slotCells;
-    a.maxU = maxU;
-    a.counts = h->counts;
-    a.fresh = h->fresh;
-    a.dead = h->dead;
-    a.totals = h->totals;
-    a.partials = h->partials;
-    a.dFluid = h->dOut;
-    a.dDead = h->dOut + LBM_MAX_SPHERES * 6;
-    a.tickets = h->redTickets;
-    a.rhoL = h->params.rhoL;
-    a.rhoG = h->params.rhoG;
-    a.gravity = h->params.gravity;
+  size_t shell_args_bytes() const override { return sizeof(ShellArgs<PopT>); }
+  void small_args(lbm_sim *h, int cur, void *out) override {
+    const SmallArgs<PopT> a = small(h, cur);
     memcpy(out, &a, sizeof(a));
   }
-  void batch_pre(const void *d_small, int n, unsigned retagCtas, unsigned compactCtas, cudaStream_t st) override {
-    const auto *A = (const SmallArgs<PopT> *)d_small;
-    kb_plan<PopT><<<n, 32, 0, st>>>(A);
-    kb_retag_box<PopT><<<dim3(retagCtas, n), 256, 0, st>>>(A);
-    kb_compact_count<PopT><<<dim3(compactCtas, n), COMPACT_THREADS, 0, st>>>(A);
-    kb_compact_scan<PopT><<<n, 1024, 0, st>>>(A);
-    kb_compact_emit<PopT><<<dim3(compactCtas, n), COMPACT_THREADS, 0, st>>>(A);
-    kb_fresh_fill<PopT><<<n, FILL_THREADS, 0, st>>>(A);
+  void shell_args(lbm_sim *h, const StepCtx &c, int cur, void *out) override {
+    const ShellArgs<PopT> a = make_shell(h, c, cur);
+    memcpy(out, &a, sizeof(a));
   }
-  void batch_post(const void *d_small, int n, int redChunks, int maxSpheres, cudaStream_t st) override {
-    if (maxSpheres <= 0) return;
-    const auto *A = (const SmallArgs<PopT> *)d_small;
-    kb_impulse_reduce<PopT><<<dim3(redChunks, maxSpheres, n), RED_THREADS, 0, st>>>(A);
-    kb_absorb_dead<PopT><<<dim3(maxSpheres, n), DEAD_THREADS, 0, st>>>(A);
-    kb_sphere_step<PopT><<<n, 32, 0, st>>>(A);
+  void batch_plan(const void *d_shell, int n, cudaStream_t st) override {
+    kb_plan<PopT><<<n, 32, 0, st>>>((const ShellArgs<PopT> *)d_shell);
+  }
+  void batch_sets(const void *d_small, int n, unsigned ctas, cudaStream_t st) override {
+    kb_sets<PopT><<<dim3(ctas, n), SETS_THREADS, 0, st>>>((const SmallArgs<PopT> *)d_small);
+  }
+  void batch_shell(const void *d_shell, int n, int redChunks, int spheres, cudaStream_t st) override {
+    kb_shell<PopT><<<dim3(redChunks, std::max(1, spheres), n), SHELL_THREADS, 0, st>>>(
+        (const ShellArgs<PopT> *)d_shell);
   }
   void warm(int device) override {
     static const int shapes[] = {2, 4, 8, 4 | LBM_FUSED_COMPACT, 6 | LBM_FUSED_COMPACT, 4 | LBM_FUSED_ASYNC,
@@ -635,11 +556,6 @@ class Ops final : public OpsBase {
     if (!Codec<PopT>::offset) return;
     k_reencode_h<PopT><<<nblocks(h->n, 256), 256, 0, h->stream>>>(scene(h), half,
                                                                     (const Real *)d_oldPhi);
-    h->launches++;
-  }
-  void sphere_step_device(lbm_sim *h, lbm_sphere *d_sph, int nsph, double gravity,
-                          const double *d_fluid, const double *d_dead) override {
-    k_sphere_step<<<1, 32, 0, h->stream>>>(d_sph, nsph, gravity, d_fluid, d_dead, h->nx, h->ny, h->nz);
     h->launches++;
   }
 };

@@ -31,6 +31,16 @@ constexpr int SHAPE_WIDE = 0x200;
 inline bool needs_wide(long long cells) { return pop_elems(cells, 27) >= (1LL << 31) - 64; }
 
 
+// A step's shell launch (lbm_shell.cuh): the step's spheres, the 1,024-cell
+// chunks of the largest one's box, and in the device-resident loop (tail) the
+// sphere step and the next plan, with slotCells impulse slots per sphere and
+// retag boxes of at most maxU cells.
+struct StepCtx {
+  int ns = 0, redChunks = 0;
+  bool tail = false;
+  long long slotCells = 0, maxU = 0;
+};
+
 class OpsBase {
  public:
   virtual ~OpsBase() {}
@@ -51,10 +61,11 @@ class OpsBase {
   virtual void stream_phase(lbm_sim *h) = 0;
   virtual void collide_hydro(lbm_sim *h) = 0;
   virtual void stream_hydro_macro(lbm_sim *h) = 0;
-  virtual void retag_box(lbm_sim *h, long long maxCells) = 0;
-  virtual void fresh_fill(lbm_sim *h) = 0;
+  // retag on the plan's box (retag), fresh / dead lists, fresh fill (fill)
+  virtual void sets(lbm_sim *h, long long maxChunks, bool retag, bool fill) = 0;
   virtual void absorb_dead(lbm_sim *h, double *d_out) = 0;
   virtual void fused_step(lbm_sim *h, const FusedCfg &cfg) = 0;
+  virtual void shell(lbm_sim *h, const StepCtx &c) = 0;  // after fused_step, before cur flips
   virtual void pack(lbm_sim *h, uint8_t *d_out) = 0;
   virtual void pack_end_planes(lbm_sim *h, uint8_t *d_out) = 0;
   virtual void watch_finite(lbm_sim *h, unsigned long long *d_first) = 0;
@@ -68,8 +79,6 @@ class OpsBase {
                                long long cells) = 0;
   // Re-express h offsets after phi changed from d_oldPhi (both halves).
   virtual void reencode_h(lbm_sim *h, int half, const void *d_oldPhi) = 0;
-  virtual void sphere_step_device(lbm_sim *h, lbm_sphere *d_sph, int nsph, double gravity,
-                                  const double *d_fluid, const double *d_dead) = 0;
   // Fused-step kernel geometry (for the bench and the autotuner).
   virtual size_t fused_smem(int ty) const = 0;
   // Batched fused step: per-scene descriptors (FusedArgs of this storage type,
@@ -92,15 +101,16 @@ class OpsBase {
   // their copy to or from a plain array of one half (the field transfers)
   virtual bool u_in_pads() const = 0;
   virtual void u_array(lbm_sim *h, int comp, int half, void *arr, bool toScene) = 0;
-  // a batch's sparse kernels, one launch per kind for all scenes: the
-  // per-scene argument block, then the kernels before and after the fused
-  // launch over a device table of n such blocks
+  // a batch's sparse work, one launch per kind for all scenes: the per-scene
+  // argument blocks, the first plans, then per step the retag, fresh / dead
+  // sets and fresh fill before the fused launch and the shells after it
   virtual size_t small_args_bytes() const = 0;
-  virtual void small_args(lbm_sim *h, int cur, int ns, long long slotCells, long long maxU, int redChunks,
-                          void *out) = 0;
-  virtual void batch_pre(const void *d_small, int n, unsigned retagCtas, unsigned compactCtas,
-                         cudaStream_t st) = 0;
-  virtual void batch_post(const void *d_small, int n, int redChunks, int maxSpheres, cudaStream_t st) = 0;
+  virtual size_t shell_args_bytes() const = 0;
+  virtual void small_args(lbm_sim *h, int cur, void *out) = 0;
+  virtual void shell_args(lbm_sim *h, const StepCtx &c, int cur, void *out) = 0;
+  virtual void batch_plan(const void *d_shell, int n, cudaStream_t st) = 0;
+  virtual void batch_sets(const void *d_small, int n, unsigned ctas, cudaStream_t st) = 0;
+  virtual void batch_shell(const void *d_shell, int n, int redChunks, int spheres, cudaStream_t st) = 0;
   // the tensor maps of the TMA-staged form (h->dMaps), where the storage
   // form and the grid allow them (nx a multiple of 16); none otherwise
   virtual int build_stage_maps(lbm_sim *) { return 0; }
@@ -136,7 +146,8 @@ struct lbm_sim {
 
   int *fresh = nullptr, *dead = nullptr;  // scan-ordered lists
   long long listCap = 0;
-  int2 *counts = nullptr;
+  int2 *counts = nullptr;  // per compaction chunk
+  void *setBits = nullptr; // per compaction chunk: its fresh / dead ballot words
   long long countsCap = 0;
   int *totals = nullptr;  // device [3]: n_fresh, n_dead, fused-step status (non-zero: a bounded wait ran out)
   bool listsValid = false;
@@ -147,14 +158,15 @@ struct lbm_sim {
   void *dMaps = nullptr;    // tensor maps of the TMA-staged form (device memory), or null
   void *meshTri = nullptr;  // a mesh's triangles for lbm_voxelize_mesh / lbm_retag_cells_mesh
   size_t meshCap = 0;
-  unsigned *redTickets = nullptr;  // [LBM_MAX_SPHERES] last-block tickets of the impulse reduction
+  unsigned *redTickets = nullptr;  // last-block tickets: [LBM_MAX_SPHERES] of the impulse sums, one of the sets kernel
   long long partialsCap = 0;  // doubles
   int partialsChunks = 0;
   double *dOut = nullptr;      // device [2][MAX][6]: fluid impulses, dead impulses
   double *hOut = nullptr;      // pinned host mirror
   lbm_sphere *dSph = nullptr;  // device sphere array for the coupled loop
   lbm::Plan hPlan{};           // host copy of the step plan
-  lbm::Plan *dPlan = nullptr;  // device step plan read by the kernels
+  lbm::Plan *dPlan = nullptr;  // [2] device step plans: the step that reads half c uses plan c
+  lbm::Plan *plan() const { return dPlan + cur; }
   void *staging = nullptr;
   size_t stagingBytes = 0;
   void *image = nullptr;  // rendered RGBA8 frame (lbm_render)
@@ -195,6 +207,7 @@ struct lbm_sim {
   // test hook: fill fresh cells with one thread in list order
   bool sequentialFill = false;
   int stepBegunNs = -1;
+  bool planOfStep = false;  // the device plan is the begun step's
   int fullRetagSteps = 0;
   int nsphLast = 0;
 
