@@ -289,6 +289,27 @@ int launch_sets(lbm_sim *h, long long maxChunks, bool retag, bool fill) {
   return LBM_OK;
 }
 
+// The z-chunk length auto_zchunk gives for the fused launch of these scenes in
+// the shape of the first (each scene's chunks evened out).
+int default_zchunk(lbm_sim *const *sims, int n) {
+  const lbm_sim *h0 = sims[0];
+  int sms = 148, planes = 1;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h0->device) != cudaSuccess) cudaGetLastError();
+  const int rows = shape_rows(h0->cfg.ty);
+  // FP64 keeps one CTA of the plain form on an SM (127 KB of ring), the compact forms two
+  const int perSM = h0->ops->macro_bytes() == 8 ? 1 : 2;
+  for (int s = 0; s < n; s++) planes = std::max(planes, sims[s]->nz - 2);
+  return auto_zchunk(planes, h0->ops->pop_bytes() == 4 ? 22 : 24, perSM, sms, [&](int zc) {
+    long long t = 0;
+    for (int s = 0; s < n; s++) {
+      const lbm_sim *h = sims[s];
+      const int len = even_zchunk(h->nz - 2, zc);
+      t += (long long)((h->nx + 31) / 32) * ((h->ny + rows - 1) / rows) * ((h->nz - 2 + len - 1) / len);
+    }
+    return t;
+  });
+}
+
 // The fused step kernel, bracketed by CUDA events when timing is on.
 void launch_fused(lbm_sim *h) {
   if (h->timing) {
@@ -700,14 +721,11 @@ int lbm_create(int nx, int ny, int nz, int storage, int device, lbm_sim **out) {
   h->n = (long long)nx * ny * nz;
   h->fusedOK = h->n < (1LL << 31) - 64;  // cell indices are 32-bit in the fused kernel
   // default launch shape: the compact-ring 6-row form with tensor prefetches
-  // into L2 (the plain compact form where nx is not a multiple of 16) in
-  // z-chunks of 22 planes (FP32) or 24 (FP16, BF16), the fastest measured at
-  // 256^3, where the storage form has it (FP32 values in the ring); the
-  // plain 4-row form for FP64
-  if (ops->shape_ok(6 | LBM_FUSED_L2PF)) {
-    h->cfg.ty = 6 | LBM_FUSED_L2PF;
-    h->cfg.zchunk = ops->pop_bytes() == 4 ? 22 : 24;
-  }
+  // into L2 (the plain compact form where nx is not a multiple of 16), the
+  // fastest measured at 256^3, where the storage form has it (FP32 values in
+  // the ring); the plain 4-row form for FP64; z-chunks by the grid
+  if (ops->shape_ok(6 | LBM_FUSED_L2PF)) h->cfg.ty = 6 | LBM_FUSED_L2PF;
+  h->cfg.zchunk = default_zchunk(&h, 1);
   h->params = lbm_params{0.6, 0.7, 0.012, 0.0010, 1.0, 0.05, 4.0, 0.02};  // src/sim.js:88-95
   int rc = LBM_OK;
   auto body = [&]() -> int {
@@ -1724,6 +1742,7 @@ int lbm_set_fused_config(lbm_sim *h, int rows, int zchunk) {
     return fail(h, LBM_ERR_ARG, "that row count needs more than 227 KB of shared memory");
   h->cfg.ty = rows;
   h->cfg.zchunk = zchunk;
+  h->cfg.set = true;
   return LBM_OK;
 }
 
@@ -1806,7 +1825,7 @@ int lbm_get_fused_config(const lbm_sim *h, int *rows, int *zchunk) {
 struct lbm_batch {
   std::vector<lbm_sim *> sims;
   int device = 0, storage = 0;
-  int rows = 4, zchunk = 32;
+  int rows = 4, zchunk = 32;  // zchunk 0: by the scenes' sizes
   std::string err;
   cudaStream_t origin = nullptr;
   cudaEvent_t fork = nullptr;
@@ -1849,6 +1868,16 @@ int bcuda(lbm_batch *b, const char *what, cudaError_t e) {
     if (rc_ != LBM_OK) return bfail(b, rc_, std::string("scene: ") + (h)->err); \
   } while (0)
 
+// z planes per CTA of each scene: the configured length, or evened-out chunks
+// of the length that suits the whole batch.
+std::vector<int> batch_zchunks(const lbm_batch *b) {
+  std::vector<int> z(b->sims.size(), b->zchunk);
+  if (b->zchunk > 0) return z;
+  const int zc = default_zchunk(b->sims.data(), (int)b->sims.size());
+  for (size_t s = 0; s < z.size(); s++) z[s] = even_zchunk(b->sims[s]->nz - 2, zc);
+  return z;
+}
+
 // Per-scene descriptors for both ping-pong parities and the tile table.
 int batch_tables(lbm_batch *b) {
   const int n = (int)b->sims.size();
@@ -1857,12 +1886,13 @@ int batch_tables(lbm_batch *b) {
   std::vector<unsigned char> args(2 * n * ab);
   std::vector<int> start(n + 1, 0);
   std::vector<int3> grid(n);
+  const std::vector<int> zc = batch_zchunks(b);
   for (int s = 0; s < n; s++) {
     lbm_sim *h = b->sims[s];
-    for (int p = 0; p < 2; p++) ops->fused_args(h, h->cur ^ p, b->zchunk, &args[(p * n + s) * ab]);
+    for (int p = 0; p < 2; p++) ops->fused_args(h, h->cur ^ p, zc[s], &args[(p * n + s) * ab]);
     const int rows = shape_rows(b->rows);
     grid[s] = make_int3((h->nx + 31) / 32, (h->ny + rows - 1) / rows,
-                        (h->nz - 2 + b->zchunk - 1) / b->zchunk);
+                        (h->nz - 2 + zc[s] - 1) / zc[s]);
     long long t = (long long)start[s] + (long long)grid[s].x * grid[s].y * grid[s].z;
     if (t > (1LL << 30)) return bfail(b, LBM_ERR_CAPACITY, "too many tiles in one batch");
     start[s + 1] = (int)t;
@@ -1908,10 +1938,13 @@ int launch_shape(const lbm_batch *b, int rows) {
 }
 
 int batch_tiles(const lbm_batch *b) {
+  const std::vector<int> zc = batch_zchunks(b);
   long long t = 0;
-  for (lbm_sim *h : b->sims)
+  for (size_t s = 0; s < zc.size(); s++) {
+    const lbm_sim *h = b->sims[s];
     t += (long long)((h->nx + 31) / 32) * ((h->ny + shape_rows(b->rows) - 1) / shape_rows(b->rows)) *
-         ((h->nz - 2 + b->zchunk - 1) / b->zchunk);
+         ((h->nz - 2 + zc[s] - 1) / zc[s]);
+  }
   return (int)t;
 }
 
@@ -1933,7 +1966,7 @@ int lbm_batch_create(lbm_sim *const *sims, int n, lbm_batch **out) {
   b->device = sims[0]->device;
   b->storage = sims[0]->storage;
   b->rows = sims[0]->cfg.ty;
-  b->zchunk = sims[0]->cfg.zchunk;
+  b->zchunk = sims[0]->cfg.set ? sims[0]->cfg.zchunk : 0;
   DeviceGuard g(b->device);
   cudaError_t e = cudaStreamCreateWithFlags(&b->origin, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);

@@ -21,7 +21,50 @@ struct FusedCfg {
   int ty = 4;       // tile shape: cell rows per CTA (CTA = 32 x (rows + 2) threads),
                     // | LBM_FUSED_COMPACT / _ASYNC / _STAGED / _TMA for the compact-ring forms
   int zchunk = 32;  // z planes marched per CTA
+  bool set = false; // by the caller (else auto_zchunk's)
 };
+
+// z planes per CTA for a launch of tiles(z) CTAs, each of which collides two
+// planes more than it writes, on `sms` SMs of which each holds `perSM` CTAs.
+// The cost of a choice is its planes per CTA times the waves of CTAs, in the
+// time a plane takes on a full SM:
+//   * one CTA on an SM takes 0.65 of that a plane (measured 2.1 us alone
+//     against 3.2 us for two, 6 compact rows);
+//   * up to two waves the last wave counts whole;
+//   * of more waves it counts a quarter of what it is short, since the CTAs
+//     are no longer in step by then;
+//   * from eight waves on only the two extra planes are left, and chunks
+//     longer than zmany read apart from their neighbours: zmany (22 planes
+//     FP32, 24 FP16 at 256^3, 14 waves, the best of 16 to 32).
+// Measured step without spheres, before (z-chunks of 22 / 24) and with the
+// rule: 40x28x40 44.7 -> 13.3 us (3 planes), 61x47x83 51.0 -> 23.8 (5),
+// 80x72x96 66.9 -> 48.7 (12), 128x97x110 FP16 110.0 -> 98.9 (27), 160x112x160
+// 201.2 -> 191.4 (27); against the best of every length the rule is within 9%
+// from 12^3 to 192x160x176.
+template <class Tiles>
+inline int auto_zchunk(int planes, int zmany, int perSM, int sms, Tiles &&tiles) {
+  constexpr int ZMAX = 32;
+  const double slots = (double)perSM * sms, alone = perSM > 1 ? 0.65 : 1.0;
+  if (tiles(zmany) >= 8 * slots) return zmany;
+  int best = 1;
+  double least = 0;
+  for (int z = 1; z <= planes && z <= ZMAX; z++) {
+    const double n = (double)tiles(z), w = n / slots, f = w - (long long)w;
+    double eff;
+    if (n <= sms) eff = alone;
+    else if (w <= 1) eff = 1;
+    else if (w < 2) eff = 1 + (f <= 0.5 ? alone : 1);
+    else eff = f > 0 ? w + 0.25 * (1 - f) : w;
+    const double cost = (z + 2) * eff;
+    if (z == 1 || cost <= least) best = z, least = cost;
+  }
+  return best;
+}
+// equal chunks of at most zmax planes
+inline int even_zchunk(int planes, int zmax) {
+  const int chunks = (planes + zmax - 1) / zmax;
+  return chunks > 0 ? (planes + chunks - 1) / chunks : 1;
+}
 
 // cell rows per CTA of a tile shape
 inline int shape_rows(int shape) { return shape & 0xff; }
