@@ -329,6 +329,15 @@ void launch_fused(lbm_sim *h) {
   }
 }
 
+// before a fused step: SOLID cells the same in both halves
+int ready_solid(lbm_sim *h) {
+  if (!h->carrySolid) return LBM_OK;
+  h->ops->carry_solid(h);
+  CKL("SOLID cells");
+  h->carrySolid = false;
+  return LBM_OK;
+}
+
 void set_box(lbm_sim *h, const Box &bx) {
   h->hPlan.U = bx;
   h->hPlan.ucells = box_cells(bx);
@@ -575,6 +584,7 @@ int coupled_prepare(lbm_sim *h, const lbm_sphere *sp, int ns, bool frames, Coupl
   c.maxChunks = (c.maxU + COMPACT_CHUNK - 1) / COMPACT_CHUNK;
   c.redChunks = (int)((c.slotCells + RED_CHUNK - 1) / RED_CHUNK);
   c.tail = true;
+  if ((rc = ready_solid(h))) return rc;
   if ((rc = ensure_work(h, std::max(1LL, (long long)ns * c.slotCells * 6),
                         (long long)std::max(ns, 1) * c.redChunks * 6)))
     return rc;
@@ -854,6 +864,7 @@ int lbm_upload_field(lbm_sim *h, int field, const void *host, size_t count) {
   if (field < 0 || field >= LBM_FIELD_COUNT) return fail(h, LBM_ERR_ARG, "unknown field");
   if (count != field_count(h, field)) return fail(h, LBM_ERR_ARG, "element count mismatch");
   EntryGuard g(h);
+  h->carrySolid = true;
   const float *src = (const float *)host;
   size_t n = (size_t)h->n;
   switch (field) {
@@ -1067,6 +1078,7 @@ static int need_phases(lbm_sim *h) {
   if (!h->ops->phases_supported())
     return fail(h, LBM_ERR_UNSUPPORTED,
                 "phase-by-phase entry points need FP32 or FP64 storage; FP16/BF16 run lbm_step only");
+  h->carrySolid = true;  // the phases work in one half
   return ensure_phase_scratch(h);
 }
 
@@ -1316,6 +1328,7 @@ int lbm_step_begin(lbm_sim *h, const lbm_sphere *sp, int ns) {
     h->stepBegunNs = ns;
     return LBM_OK;
   }
+  if ((rc = ready_solid(h))) return rc;
   if ((rc = set_solids(h, sp, ns, true))) return rc;
   Box now = spheres_box(h, sp, ns);
   Box U;
@@ -1757,6 +1770,7 @@ int lbm_set_slab(lbm_sim *h, int zoff, int own_lo, int own_hi) {
   h->ownLo = own_lo;
   h->ownHi = own_hi;
   h->fullRetagSteps = 2;
+  h->carrySolid = true;
   return LBM_OK;
 }
 
@@ -1801,6 +1815,7 @@ int lbm_slab_copy_planes(lbm_sim *dst, int dst_plane, const lbm_sim *src, int sr
   CK(copy(dst->tag + dc, src->tag + sc, (size_t)cells));
   CK(cudaStreamSynchronize(dst->stream));
   dst->listsValid = false;
+  dst->carrySolid = true;
   return LBM_OK;
 }
 

@@ -741,30 +741,7 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
     const int i = z * nxny + y * nx + x;
     const POff bF = (POff)(i >> 3) * BLK27 + (i & 7) * 4;
     const POff bH = (POff)(i >> 3) * BLK7 + (i & 7) * 4;
-    if (tagI == TAG_SOLID) {
-      // Solid cells are not updated; carry their state into the next half so
-      // both halves hold the reference's stale values.
-#pragma unroll 1
-      for (int g = 0; g < G27; g++) {
-        PopT t[4];
-        ldg4_at(Fc, bF + 32 * g, nF, 10, true, t);
-        st4_at(Fn, bF + 32 * g, nF, 10, t);
-      }
-#pragma unroll 1
-      for (int g = 0; g < G7; g++) {
-        PopT t[4];
-        ldg4_at(Hc, bH + 32 * g, nH, 11, true, t);
-        st4_at(Hn, bH + 32 * g, nH, 11, t);
-      }
-      st_at(s.phi[nxt], i, nCell, 12, ldg_at(phiC, i, nCell, 12));
-      st_at(s.rho[nxt], i, nCell, 12, ldg_at(rhoC, i, nCell, 12));
-      if constexpr (!UPAD) {  // (in the pads, copied with the groups above)
-        st_at(s.ux[nxt], i, nCell, 12, ldg_at(uxC, i, nCell, 12));
-        st_at(s.uy[nxt], i, nCell, 12, ldg_at(uyC, i, nCell, 12));
-      }
-      st_at(s.uz[nxt], i, nCell, 12, ldg_at(uzC, i, nCell, 12));
-      if (PACK && lbm_ok(i < nCell, 50, i)) pack_rg8(a.pack, i, ldg_at(phiC, i, nCell, 12), true);
-    } else if (tagI == TAG_FLUID) {
+    if (tagI == TAG_FLUID) {
       // ring copies: group e_z sources come from plane z - e_z; the cell's own
       // (bounce-back) values are in plane z
       const int zMs = ring_copy<CM>(z + 1), zMo = ring_copy<CM>(z), zZ = ring_copy<CZ>(z);
@@ -872,9 +849,9 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
       st_at(s.uz[nxt], i, nCell, 18, uzn);
       if (PACK && lbm_ok(i < nCell, 50, i)) pack_rg8(a.pack, i, p, false);
     } else if (PACK && cellWarp && x < nx && y < ny && z >= zb) {
-      // a wall cell of this tile: not updated, packed from the half that is
-      // current after the step
-      if (lbm_ok(i < nCell, 50, i)) pack_rg8(a.pack, i, ldg_at(s.phi[nxt], i, nCell, 12), false);
+      // a wall or SOLID cell of this tile: not updated, packed from the half that
+      // is current after the step
+      if (lbm_ok(i < nCell, 50, i)) pack_rg8(a.pack, i, ldg_at(s.phi[nxt], i, nCell, 12), tagI == TAG_SOLID);
     }
     gxC = gxN;
     gyC = gyN;

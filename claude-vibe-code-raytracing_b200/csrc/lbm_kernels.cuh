@@ -543,6 +543,41 @@ __device__ __forceinline__ void fresh_fill_body(const Scene<PopT, typename Prec<
     if (!__syncthreads_or(waiting)) break;
   }
 }
+// ---------------------------------------------------------------- SOLID cells
+// The step updates FLUID cells only; a SOLID cell keeps its values in both
+// halves.  It gets them into the half that the step writes when it turns SOLID
+// (k_sets), and the tiles pass it by: copying every SOLID cell in every step
+// made the warps inside a sphere wait nine memory latencies a plane (160x112x160
+// with one sphere 227 -> 193 us a launch on a B200).
+template <class PopT>
+__device__ __forceinline__ void carry_cell(const Scene<PopT, typename Prec<PopT>::Real> &s, int cur, long long i) {
+  using Real = typename Prec<PopT>::Real;
+  struct alignas(4 * sizeof(PopT) > 16 ? 16 : 4 * sizeof(PopT)) Group {
+    PopT v[4];
+  };
+  const int nxt = 1 - cur;
+  Group f[PopGroups<Q27>::G], h[PopGroups<Q7>::G];
+  const long long F = pidx<27>(0, i), H = pidx<7>(0, i);
+  for (int g = 0; g < PopGroups<Q27>::G; g++) f[g] = *reinterpret_cast<const Group *>(s.F[cur] + F + 32 * g);
+  for (int g = 0; g < PopGroups<Q7>::G; g++) h[g] = *reinterpret_cast<const Group *>(s.H[cur] + H + 32 * g);
+  const Real p = s.phi[cur][i], r = s.rho[cur][i], z = s.uz[cur][i];
+  for (int g = 0; g < PopGroups<Q27>::G; g++) *reinterpret_cast<Group *>(s.F[nxt] + F + 32 * g) = f[g];
+  for (int g = 0; g < PopGroups<Q7>::G; g++) *reinterpret_cast<Group *>(s.H[nxt] + H + 32 * g) = h[g];
+  s.phi[nxt][i] = p;
+  s.rho[nxt][i] = r;
+  s.uz[nxt][i] = z;
+  if constexpr (!Scene<PopT, Real>::UPAD) {  // (in the pads, copied with the groups)
+    s.ux[nxt][i] = s.ux[cur][i];
+    s.uy[nxt][i] = s.uy[cur][i];
+  }
+}
+// every SOLID cell of the grid, after calls that may have changed one half alone
+template <class PopT>
+__global__ void k_carry_solid(Scene<PopT, typename Prec<PopT>::Real> s, int cur) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < s.n; i += (long long)gridDim.x * blockDim.x)
+    if (s.tag[i] == TAG_SOLID) carry_cell<PopT>(s, cur, i);
+}
+
 // ---------------------------------------------------------------- retag, fresh / dead sets, fresh fill
 // Arguments of a scene's sparse kernels (by value for one scene; a batch reads
 // one block per scene from device memory).
@@ -560,7 +595,8 @@ struct SmallArgs {
 
 // The first three parts of a step around the spheres in one launch: retagCells
 // on the plan's box (RETAG; src/sim.js:214-244: every cell outside the union of
-// the current and the two previous sphere boxes keeps tag == tagPrev), the
+// the current and the two previous sphere boxes keeps tag == tagPrev; a cell
+// that turns SOLID is copied into the half that the step writes), the
 // scan-ordered lists of fresh (FLUID, was SOLID) and dead (SOLID, was FLUID)
 // cells, and handleFreshCells (FILL).
 //
@@ -624,6 +660,7 @@ __device__ __forceinline__ void sets_body(const SmallArgs<PopT> &a, unsigned bid
         }
         isF = t[j] == TAG_FLUID && p[j] == TAG_SOLID;
         isD = t[j] == TAG_SOLID && p[j] == TAG_FLUID;
+        if (RETAG && isD) carry_cell<PopT>(s, a.cur, cell[j]);
       }
       const unsigned bf = __ballot_sync(0xffffffffu, isF), bd = __ballot_sync(0xffffffffu, isD);
       if (lane == 0)

@@ -216,6 +216,10 @@ class Ops final : public OpsBase {
     a.rhoG = h->params.rhoG;
     return a;
   }
+  void carry_solid(lbm_sim *h) override {
+    k_carry_solid<PopT><<<std::min(nblocks(h->n, 256), 148u * 8u), 256, 0, h->stream>>>(scene(h), h->cur);
+    h->launches++;
+  }
   void sets(lbm_sim *h, long long maxChunks, bool retag, bool fill) override {
     const unsigned ctas = (unsigned)std::min<long long>(std::max(1LL, maxChunks), SWEEP_CTAS);
     const SmallArgs<PopT> a = small(h, h->cur);
