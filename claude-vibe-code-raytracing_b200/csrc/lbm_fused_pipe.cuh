@@ -99,11 +99,10 @@ struct PipeRing {
   // Copies of each e_z group, one per plane whose slots may still be read
   // while the next plane is written.  A plane's e_z = -1 slots are read by
   // the pulls of the plane below and of itself, its e_z = 0 slots by its own
-  // pull, its e_z = +1 slots by its own pull and the plane above's, its tags
-  // by the pulls of the planes below, at and above it; a barrier separates
-  // the pull of plane q - 2 from the writes of plane q, so 2 / 2 / 3 copies
-  // and 3 tag planes suffice.
-  static constexpr int CM = 2, CZ = 2, CP = 3, CT = 3;
+  // pull, its e_z = +1 slots by its own pull and the plane above's; a barrier
+  // separates the pull of plane q - 2 from the writes of plane q, so 2 / 2 / 3
+  // copies suffice.
+  static constexpr int CM = 2, CZ = 2, CP = 3;
   // f: e_z = -1 group in CM copies, e_z = 0 in CZ, e_z = +1 in CP; h likewise
   static constexpr int FM = 0;
   static constexpr int FZ = FM + CM * grp(27, -1);
@@ -129,8 +128,7 @@ struct PipeSmem {
   using Real = typename Prec<PopT>::Real;
   static constexpr bool STG = PF == PIPE_STAGED, ASY = PF == PIPE_ASYNC, TMA = PF == PIPE_TMA;
   using R = PipeRing<TY>;
-  static constexpr int CT = R::CT;  // tag planes
-  static constexpr int RX = 34, RY = TY + 2, NC = RX * RY;  // tag planes keep the full halo frame
+  static constexpr int RX = 34, RY = TY + 2, NC = RX * RY;  // the tags keep the full halo frame
   // blocks a 32-cell row can span (4 when rows start on a block: TMA)
   static constexpr int SB = TMA ? 4 : 5;
   static constexpr int ROWF = SB * PopGroups<Q27>::BLOCK, ROWH = SB * PopGroups<Q7>::BLOCK;
@@ -145,7 +143,7 @@ struct PipeSmem {
   static constexpr size_t lead = TMA ? 128 : 0;  // room to align the base up
   static constexpr size_t ringBytes = (size_t)R::TOTAL * sizeof(Real);
   static constexpr size_t tagOff = ringBytes;
-  static constexpr size_t stF = (tagOff + CT * NC + AL - 1) / AL * AL;
+  static constexpr size_t stF = (tagOff + 4 * NC + AL - 1) / AL * AL;
   static constexpr size_t stH = stF + (size_t)TY * ROWF * sizeof(PopT);
   static constexpr size_t stM = stH + (size_t)TY * ROWH * sizeof(PopT);
   static constexpr size_t stT = stM + (size_t)4 * TY * MROW * sizeof(Real);
@@ -162,7 +160,7 @@ struct PipeSmem {
   // groups of f, [G7][32 TY] groups of h, [11][32 TY] words (phi and its six
   // neighbours, rho, ux, uy, uz)
   static constexpr int NT = 32 * TY, GB = 4 * (int)sizeof(PopT), NS = 11;
-  static constexpr size_t aF = (tagOff + CT * NC + 15) / 16 * 16;
+  static constexpr size_t aF = (tagOff + 4 * NC + 15) / 16 * 16;
   static constexpr size_t aH = aF + (size_t)PopGroups<Q27>::G * NT * GB;
   static constexpr size_t aS = aH + (size_t)PopGroups<Q7>::G * NT * GB;
   // staged: two mbarriers (stage full, stage read) and the abort flag (TMA:
@@ -196,10 +194,10 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
   using SM = PipeSmem<PopT, TY, PF>;
   constexpr bool STG = SM::STG, ASY = SM::ASY, TMA = SM::TMA, L2P = PF == PIPE_L2PF;
   using R = PipeRing<TY>;
-  constexpr int CM = R::CM, CZ = R::CZ, CP = R::CP, CT = R::CT;
+  constexpr int CM = R::CM, CZ = R::CZ, CP = R::CP;
   using LD = CellLoad<PopT>;
   using CO = CellOut<PopT>;
-  constexpr int RX = SM::RX, NC = SM::NC, TAGS = CT * NC, RING = R::TOTAL;
+  constexpr int RX = SM::RX, NC = SM::NC, RING = R::TOTAL;
   constexpr int G27 = PopGroups<Q27>::G, G7 = PopGroups<Q7>::G;
   constexpr int BLK27 = PopGroups<Q27>::BLOCK, BLK7 = PopGroups<Q7>::BLOCK;
   constexpr int ROWF = SM::ROWF, ROWH = SM::ROWH, MROW = SM::MROW, TROW = SM::TROW, PROW = SM::PROW;
@@ -208,7 +206,7 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
   unsigned char *smem = smem_raw;
   if constexpr (SM::lead > 0) smem += (SM::lead - (smem_u32(smem_raw) & (SM::lead - 1))) & (SM::lead - 1);
   Real *ring = reinterpret_cast<Real *>(smem);
-  uint8_t *stag = smem + SM::tagOff;                           // [3][NC]
+  uint32_t *stag = reinterpret_cast<uint32_t *>(smem + SM::tagOff);  // [NC] three planes' tags of a cell
   PopT *sF = reinterpret_cast<PopT *>(smem + SM::stF);         // [TY][ROWF]
   PopT *sH = reinterpret_cast<PopT *>(smem + SM::stH);         // [TY][ROWH]
   Real *sM = reinterpret_cast<Real *>(smem + SM::stM);         // [4][TY][MROW] rho ux uy uz
@@ -533,6 +531,10 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
     L.tg = tg;
   };
 
+  // The tags of a cell in the three planes collided last, the latest in the low
+  // byte: one word per cell, so a pull reads nine words instead of 27 bytes.
+  uint32_t tags = 0, tags2 = 0;  // (the row warp's second cell)
+
   // ---- emit: collided values and tag of a cell into the ring (local cell lx, ly)
   auto emit = [&](auto MODEc, auto SXc, auto SYc, int sx, int sy, bool active, int q, int lx, int ly,
                   const CO &o) __attribute__((always_inline)) {
@@ -543,7 +545,9 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
     const int hM = R::HM + qM * R::grp(7, -1), hZ = R::HZ + qZ * R::grp(7, 0);
     const int hP = R::HP + qP * R::grp(7, 1);
     const int lc = (ly + 1) * RX + (lx + 1);
-    if (MODE != 2 || active) stag[sm_at(ring_copy<CT>(q) * NC + lc, TAGS, 2)] = (MODE == 1 && SY < 0) ? o.tg2 : o.tg;
+    uint32_t &h = (MODE == 1 && SY < 0) ? tags2 : tags;
+    h = h << 8 | ((MODE == 1 && SY < 0) ? o.tg2 : o.tg);
+    if (MODE != 2 || active) stag[sm_at(lc, NC, 2)] = h;
     static_for<0, Q27>([&](auto KK) {
       constexpr int k = decltype(KK)::value;
       constexpr int ez = kDir[k][2];
@@ -762,8 +766,7 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
 
     // pull plane z = q - 1 (nothing while z < zb)
     const int z = q - 1;
-    const int sC = ring_copy<CT>(z);
-    const uint8_t tagI = colActive && z >= zb ? stag[sm_at(sC * NC + own, TAGS, 9)] : TAG_WALL;
+    const uint8_t tagI = colActive && z >= zb ? (uint8_t)(tags >> 8) : TAG_WALL;
     const int i = z * nxny + y * nx + x;
     const POff bF = (POff)(i >> 3) * BLK27 + (i & 7) * 4;
     const POff bH = (POff)(i >> 3) * BLK7 + (i & 7) * 4;
@@ -778,23 +781,27 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
       const int sHM = R::HM + zMs * R::grp(7, -1), sHZ = R::HZ + zZ * R::grp(7, 0);
       const int sHP = R::HP + zPs * R::grp(7, 1);
       const int oHM = R::HM + zMo * R::grp(7, -1), oHP = R::HP + zPo * R::grp(7, 1);
-      const int tbM = ring_copy<CT>(z + 1) * NC + own, tbZ = sC * NC + own, tbP = ring_copy<CT>(z - 1) * NC + own;
+      // the sources' tags: word (ex, ey) has plane z + 1, z, z - 1 in its bytes
+      uint32_t tw[3][3], orTags = 0;
+#pragma unroll
+      for (int b = 0; b < 3; b++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          tw[b][c] = stag[sm_at(own - (b - 1) * RX - (c - 1), NC, 13)];
+          orTags |= tw[b][c];
+        }
       Real rhoA = 0, mx = 0, my = 0, mz = 0, hsum = 0;
       Real hn[Q7];
       Real val4[4], ref4[4];
       PopT enc4[4], lastF[4];
-      uint32_t orTags = 0;
       static_for<0, Q27>([&](auto KK) {
         constexpr int k = decltype(KK)::value;
         using D = D27<k>;
         constexpr int ex = D::ex, ey = D::ey, ez = D::ez, o = D::opp;
         constexpr int oz = D27<o>::ez;
-        constexpr int so = -ey * RX - ex;
-        const int tb = ez < 0 ? tbM : (ez == 0 ? tbZ : tbP);
         const int sbF = ez < 0 ? sFM : (ez == 0 ? sFZ : sFP);
         const int obF = oz < 0 ? oFM : (oz == 0 ? sFZ : oFP);
-        const uint8_t ts = stag[sm_at(tb + so, TAGS, 13)];
-        const bool fl = ts == TAG_FLUID;
+        const bool fl = (tw[ey + 1][ex + 1] & (0xffu << (8 * (ez + 1)))) == 0;  // TAG_FLUID
         // source (tx - ex, ty - ey) in direction k's array; own cell in o's.
         // Both are read and the value selected, so each load keeps its
         // compile-time offset and no address is selected per direction.
@@ -807,7 +814,6 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
         const Real fO = ring[obF + r33 + R::at(27, o, 0, 0)];
         const Real fk = fl ? fS : fO;
 #endif
-        orTags |= ts;
         val4[k & 3] = fk;
         ref4[k & 3] = (Real)D::w;
         if constexpr ((k & 3) == 3 || k == Q27 - 1) {
@@ -846,7 +852,8 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
       finish_macros(K, p, gxC, gyC, gzC, lapC, rhoA, mx, my, mz, rhoN, uxn, uyn, uzn);
       // a cell next to a sphere leaves the sums themselves: the shell launch
       // adds its moving-wall links and finishes it
-      if (orTags & TAG_SOLID) rhoN = rhoA, uxn = mx, uyn = my, uzn = mz;
+      static_assert(TAG_FLUID == 0 && (TAG_SOLID & TAG_WALL) == 0, "tag bits");
+      if (orTags & (TAG_SOLID * 0x010101u)) rhoN = rhoA, uxn = mx, uyn = my, uzn = mz;
       // h, the last group's pad holding uy where u sits in the pads (the
       // FP32 / FP64 codec stores it unchanged), +0 otherwise
       static_for<0, Q7>([&](auto KK) {
