@@ -269,11 +269,24 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
     else if constexpr (MODE == 1) return active && halo_dir<SX, SY, k>();
     else return active && D27<k>::ex == SX && (sy == 0 || D27<k>::ey == sy);  // side: e_x fixed, e_y run time
   };
-  auto load = [&](auto MODEc, auto SXc, auto SYc, int sx, int sy, bool active, int q, int gx_, int gy_,
+  // A thread's cells keep their column through the planes.  Boundary cells, and
+  // those outside the grid, are walls whatever their tags say (they never act as
+  // fluid and nothing of them is read): they load an interior cell instead, so
+  // no load needs its address clamped.
+  struct Column {
+    int cell;    // of the column (or of column (1, 1)) in plane 0
+    bool inner;  // not a wall by its place
+  };
+  auto column = [&](int gx_, int gy_) __attribute__((always_inline)) -> Column {
+    const bool in = gx_ >= 1 && gx_ <= nx - 2 && gy_ >= 1 && gy_ <= ny - 2;
+    return Column{in ? gy_ * nx + gx_ : nx + 1, in};
+  };
+  const Column col = cellWarp ? column(x, y) : haloRows ? column(x, y0 - 1) : column(x0 - 1 + sideLx, y0 - 1 + sideLy);
+  const Column col2 = column(x, y0 + TY);  // (the row warp's second cell)
+  auto load = [&](auto MODEc, auto SXc, auto SYc, int sx, int sy, bool active, int q, const Column &at,
                   LD &L) __attribute__((always_inline)) {
     constexpr int MODE = decltype(MODEc)::value, SX = decltype(SXc)::value, SY = decltype(SYc)::value;
-    const bool inside = gx_ >= 0 && gx_ < nx && gy_ >= 0 && gy_ < ny && q >= 0 && q < nz;
-    const int ci = inside ? q * nxny + gy_ * nx + gx_ : 0;
+    const int ci = min(max(q, 1), nz - 2) * nxny + at.cell;
     const POff bF = (POff)(ci >> 3) * BLK27 + (ci & 7) * 4;
     const POff bH = (POff)(ci >> 3) * BLK7 + (ci & 7) * 4;
     // pad: element Q of the last group (ux for f, uy for h where they sit in
@@ -301,15 +314,14 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
     PopT padF = PopT(), padH = PopT();
     groups(IC<Q27>{}, IC<G27>{}, Fc, bF, nF, 3, L.fv, padF);
     groups(IC<Q7>{}, IC<G7>{}, Hc, bH, nH, 4, L.hv, padH);
-    uint8_t tg = ldg_at(tagA, ci, nCell, 1);
-    const int last = (int)nCell - 1;
+    const uint8_t tg = ldg_at(tagA, ci, nCell, 1);
     L.p = ldg_at(phiC, ci, nCell, 5);
-    L.pxp = ldg_at(phiC, min(ci + 1, last), nCell, 5);
-    L.pxm = ldg_at(phiC, max(ci - 1, 0), nCell, 5);
-    L.pyp = ldg_at(phiC, min(ci + nx, last), nCell, 5);
-    L.pym = ldg_at(phiC, max(ci - nx, 0), nCell, 5);
-    L.pzp = ldg_at(phiC, min(ci + nxny, last), nCell, 5);
-    L.pzm = ldg_at(phiC, max(ci - nxny, 0), nCell, 5);
+    L.pxp = ldg_at(phiC, ci + 1, nCell, 5);
+    L.pxm = ldg_at(phiC, ci - 1, nCell, 5);
+    L.pyp = ldg_at(phiC, ci + nx, nCell, 5);
+    L.pym = ldg_at(phiC, ci - nx, nCell, 5);
+    L.pzp = ldg_at(phiC, ci + nxny, nCell, 5);
+    L.pzm = ldg_at(phiC, ci - nxny, nCell, 5);
     L.sumF = ldg_at(rhoC, ci, nCell, 6);
     if constexpr (UPAD && MODE == 0) {
       // a tile cell loads every group, the pads included
@@ -323,23 +335,21 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
       L.uy = ldg_at(uyC, ci, nCell, 6);
     }
     L.uz = ldg_at(uzC, ci, nCell, 6);
-    const bool inner = gx_ >= 1 && gx_ <= nx - 2 && gy_ >= 1 && gy_ <= ny - 2 && q >= 1 && q <= nz - 2;
-    if (!inside || (!inner && tg == TAG_FLUID)) tg = TAG_WALL;
-    L.tg = tg;
+    L.tg = at.inner && q >= 1 && q <= nz - 2 ? tg : TAG_WALL;
   };
   // the row warp's two cells (above and below the tile) share one load set's
   // worth of registers each; the side warp has one cell per lane
   auto halo_load = [&](int q, LD &L, LD &L2) __attribute__((always_inline)) {
     if (haloRows) {
-      load(IC<1>{}, IC<0>{}, IC<1>{}, 0, 0, true, q, x, y0 - 1, L);
-      load(IC<1>{}, IC<0>{}, IC<-1>{}, 0, 0, true, q, x, y0 + TY, L2);
+      load(IC<1>{}, IC<0>{}, IC<1>{}, 0, 0, true, q, col, L);
+      load(IC<1>{}, IC<0>{}, IC<-1>{}, 0, 0, true, q, col2, L2);
     } else {
       // the side warp's cell, mirrored in x on the right: both halves then
       // collide the directions with e_x = +1 (the x components change sign,
       // exactly) in one pass.  As two divergent passes, each with its own load
       // latency, the side warp was what the others waited for at the barrier:
       // 256^3 FP32 1037 -> 993 us, FP16 970 -> 888, BF16 993 -> 908 (B200)
-      load(IC<0>{}, IC<0>{}, IC<0>{}, 0, 0, true, q, x0 - 1 + sideLx, y0 - 1 + sideLy, L);
+      load(IC<0>{}, IC<0>{}, IC<0>{}, 0, 0, true, q, col, L);
       static_for<0, Q27>([&](auto KK) {
         constexpr int k = decltype(KK)::value;
         if constexpr (kDir[k][0] == 1) {
@@ -711,7 +721,7 @@ __device__ __forceinline__ void fused_tile_pipe(const FusedArgs<PopT> &a, int bx
       } else if constexpr (ASY) {
         async_load(q, tgNext, L);
       } else {
-        load(IC<0>{}, IC<0>{}, IC<0>{}, 0, 0, true, q, x, y, L);
+        load(IC<0>{}, IC<0>{}, IC<0>{}, 0, 0, true, q, col, L);
       }
       collide_cell<PopT, 0, 0, 0>(K, L, o, gxN, gyN, gzN, lapN);
     } else {
