@@ -382,167 +382,134 @@ __device__ __forceinline__ void box_cell(const Box &bx, long long l, int &x, int
   z = bx.lo[2] + (int)(l / ((long long)dx * dy));
 }
 
-// One fresh cell (src/sim.js:264-308): the FLUID neighbours' phi, rho and u
-// averaged in the reference's neighbour order (dz, dy, dx ascending), then phi,
-// phiPrev, rho, u and the equilibrium populations written.  nb(j, p, r, x, y,
-// z) gives neighbour j's five values.
-template <class PopT, class NB>
-__device__ __forceinline__ void fill_cell(const Scene<PopT, typename Prec<PopT>::Real> &s, int cur, long long i,
-                                          double rhoL, double rhoG, NB &&nb) {
-  using Real = typename Prec<PopT>::Real;
-  const int nx = s.nx, ny = s.ny;
-  double psum = 0, rsum = 0, vxs = 0, vys = 0, vzs = 0;
-  int pcnt = 0;
-  for (int dz = -1; dz <= 1; dz++)
-    for (int dy = -1; dy <= 1; dy++)
-      for (int dx = -1; dx <= 1; dx++) {
-        if (!dx && !dy && !dz) continue;
-        long long j = i + ((long long)dz * ny + dy) * nx + dx;
-        // (from L2: other blocks of the same launch may have written the tag)
-        if (__ldcg(s.tag + j) == TAG_FLUID) {
-          Real vp, vr, vx_, vy_, vz_;
-          nb(j, vp, vr, vx_, vy_, vz_);
-          psum += (double)vp;
-          rsum += (double)vr;
-          vxs += (double)vx_;
-          vys += (double)vy_;
-          vzs += (double)vz_;
-          pcnt++;
-        }
-      }
-  double p = pcnt > 0 ? psum / pcnt : (double)s.phi[cur][i];
-  double r = pcnt > 0 ? rsum / pcnt : 1.0;
-  double vx = pcnt > 0 ? vxs / pcnt : 0;
-  double vy = pcnt > 0 ? vys / pcnt : 0;
-  double vz = pcnt > 0 ? vzs / pcnt : 0;
-  Real pR = (Real)p;
-  s.phi[cur][i] = pR;
-  s.phi[1 - cur][i] = pR;  // phiPrev[i] = p
-  s.rho[cur][i] = (Real)r;
-  s.set_ux(cur, i, (Real)vx);
-  s.set_uy(cur, i, (Real)vy);
-  s.uz[cur][i] = (Real)vz;
-  double rhoPhase = rhoG + p * (rhoL - rhoG);
-  double u2 = vx * vx + vy * vy + vz * vz;
-  for (int k = 0; k < Q27; k++) {
-    double eu = dcomp(k, 0) * vx + dcomp(k, 1) * vy + dcomp(k, 2) * vz;
-    double Qi = eu * (3.0 + 4.5 * eu) - 1.5 * u2;
-    double fk = (double)w27_of(k) * (r + rhoPhase * Qi);
-    s.F[cur][pidx<27>(k, i)] = Codec<PopT>::enc((Real)fk, (Real)w27_of(k));
-  }
-  for (int k = 0; k < Q7; k++) {
-    double eu = dcomp(k, 0) * vx + dcomp(k, 1) * vy + dcomp(k, 2) * vz;
-    double hk = (double)w7_of(k) * p * (1 + 4.0 * eu);
-    s.H[cur][pidx<7>(k, i)] = Codec<PopT>::enc((Real)hk, (Real)w7_of(k) * pR);
-  }
-}
+// handleFreshCells over the scan-ordered fresh list (src/sim.js:257-310): the
+// FLUID neighbours' phi, rho and u averaged in the reference's neighbour order
+// (dz, dy, dx ascending), then phi, phiPrev, rho, u and the equilibrium
+// populations written.  The reference fills in scan order, in place: a fresh
+// cell sees the filled values of fresh neighbours before it in scan order and
+// the old values of those after it.
+//
+// FILL_GROUP cells of the list at a time: a lane per neighbour stages its five
+// values, all in one memory latency; a thread per cell and value adds them in
+// neighbour order; a lane per direction writes the populations.  The order
+// between the cells of a group is kept by rounds: a cell is filled in the first
+// round in which its fresh neighbours before it have been filled.  A z slab
+// fills its own planes only (its copied planes receive the neighbouring slab's
+// filled values).  sequential != 0: one cell at a time.
+// Latency-bound: with a thread per cell that went from neighbour to neighbour,
+// one fresh cell took 31,000 cycles and twenty 75,000 to 118,000 (256^3, one
+// sphere of radius 24); now 6,600, and 10,000 to 15,000.
+constexpr int FILL_GROUP = 32;
 
-// Fresh cells a block fills in parallel; a longer list is filled by one
-// thread in list order.
-constexpr int FILL_PAR_MAX = 512;
-constexpr int FILL_THREADS = 256;
-
-// handleFreshCells over the scan-ordered fresh list (src/sim.js:257-310).  The
-// reference fills in scan order, in place: a fresh cell sees the filled values
-// of fresh neighbours before it in scan order and the old values of those
-// after it.  In parallel that order is kept by rounds: the old phi, rho and u
-// of every listed cell are saved first; in each round a cell whose fresh
-// neighbours before it in scan order were all filled in earlier rounds is
-// filled, reading the saved old values for fresh neighbours after it.  The
-// arithmetic of each cell is the sequential one (fill_cell), so the results
-// are the same bit for bit.  A z slab fills its own planes only (its copied
-// planes receive the neighbouring slab's filled values).  sequential != 0: one
-// thread in list order (also used for lists longer than FILL_PAR_MAX).
-template <class PopT>
+template <class PopT, int THREADS>
 __device__ __forceinline__ void fresh_fill_body(const Scene<PopT, typename Prec<PopT>::Real> &s, int cur,
                                                 const int *fresh, int nf, double rhoL, double rhoG, int zlo,
                                                 int zend, int sequential) {
   using Real = typename Prec<PopT>::Real;
-  const long long nxny = (long long)s.nx * s.ny;
-  auto skip = [&](long long i) -> bool {
-    if (zend <= 0) return false;
-    const long long z = i / nxny;
-    return z < zlo || z >= zend;
-  };
-  auto current = [&](long long j, Real &p, Real &r, Real &x, Real &y, Real &z) {
-    p = s.phi[cur][j];
-    r = s.rho[cur][j];
-    x = s.ux_at(cur, j);
-    y = s.uy_at(cur, j);
-    z = s.uz[cur][j];
-  };
-  if (sequential || nf > FILL_PAR_MAX) {
-    if (threadIdx.x != 0) return;
-    for (int q = 0; q < nf; q++) {
-      const long long i = fresh[q];
-      if (!skip(i)) fill_cell<PopT>(s, cur, i, rhoL, rhoG, current);
-    }
-    return;
-  }
-  __shared__ int sIdx[FILL_PAR_MAX];
-  __shared__ int sDone[FILL_PAR_MAX];  // round in which the cell was filled (or skipped), 0: not yet
-  __shared__ Real sOld[5][FILL_PAR_MAX];
-  for (int q = threadIdx.x; q < nf; q += blockDim.x) {
-    const long long i = fresh[q];
-    sIdx[q] = (int)i;
-    sDone[q] = 0;
-    current(i, sOld[0][q], sOld[1][q], sOld[2][q], sOld[3][q], sOld[4][q]);
-  }
-  __syncthreads();
-  // list position of cell j, or -1 (the list is sorted by cell index)
-  auto find = [&](long long j) -> int {
-    int lo = 0, hi = nf - 1;
-    while (lo <= hi) {
-      const int mid = (lo + hi) >> 1;
-      const int v = sIdx[mid];
-      if (v == j) return mid;
-      if (v < j) lo = mid + 1;
-      else hi = mid - 1;
-    }
-    return -1;
-  };
-  for (int round = 1;; round++) {
-    int waiting = 0;
-    for (int q = threadIdx.x; q < nf; q += blockDim.x) {
-      if (sDone[q]) continue;
-      const long long i = sIdx[q];
-      if (skip(i)) {
-        sDone[q] = round;
-        continue;
+  constexpr int WARPS = THREADS / 32, OWN = 13;  // (neighbour 13 is the cell itself)
+  static_assert(FILL_GROUP == 32 && FILL_GROUP % WARPS == 0 && THREADS >= 5 * FILL_GROUP, "");
+  __shared__ Real sVal[FILL_GROUP][5][Q27];  // phi, rho, u of the neighbours (0 where not FLUID) and the cell's own
+  __shared__ double sMean[FILL_GROUP][5];
+  __shared__ int sRaw[FILL_GROUP], sIdx[FILL_GROUP];  // the cell; -1 where it is another slab's
+  __shared__ int sCnt[FILL_GROUP];                    // its FLUID neighbours
+  __shared__ uint32_t sNeed[FILL_GROUP], sDone;       // cells of the group it waits for; those filled
+  __shared__ int8_t sDep[FILL_GROUP][OWN];            // place in the group of each neighbour before it, or -1
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nxny = s.nx * s.ny;
+  const int dz = lane / 9 - 1, dy = lane / 3 % 3 - 1, dx = lane % 3 - 1;
+  const int k = min(lane, Q27 - 1);  // the lane's direction
+  const double ex = dcomp(k, 0), ey = dcomp(k, 1), ez = dcomp(k, 2);
+  const float w = w27_of(k), w7 = w7_of(min(k, Q7 - 1));
+  const int group = sequential ? 1 : FILL_GROUP;
+  for (int g0 = 0; g0 < nf; g0 += group) {
+    const int m = min(group, nf - g0);
+    if (threadIdx.x < FILL_GROUP) {
+      int i = -1;
+      if (lane < m) {
+        i = sRaw[lane] = fresh[g0 + lane];
+        const int z = i / nxny;
+        if (zend > 0 && (z < zlo || z >= zend)) i = -1;
       }
-      bool ready = true;
-      for (int dz = -1; dz <= 0 && ready; dz++)
-        for (int dy = -1; dy <= 1 && ready; dy++)
-          for (int dx = -1; dx <= 1; dx++) {
-            if (dz == 0 && (dy > 0 || (dy == 0 && dx >= 0))) break;  // only neighbours before i
-            const long long j = i + ((long long)dz * s.ny + dy) * s.nx + dx;
-            const int pos = find(j);
-            if (pos >= 0 && (sDone[pos] == 0 || sDone[pos] >= round)) {
-              ready = false;
-              break;
-            }
-          }
-      if (!ready) {
-        waiting = 1;
-        continue;
+      sIdx[lane] = i;
+      sNeed[lane] = 0;
+      if (lane == 0) sDone = 0;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int e = threadIdx.x; e < m * OWN; e += THREADS) {
+      const int q = e / OWN, n = e - q * OWN, i = sIdx[q];
+      const int j = i + (n / 9 - 1) * nxny + (n / 3 % 3 - 1) * s.nx + n % 3 - 1;
+      int lo = 0, hi = q - 1, dep = -1;  // (the list is sorted by cell index)
+      while (lo <= hi) {
+        const int mid = (lo + hi) >> 1, at = sRaw[mid];
+        if (at == j) dep = mid;
+        if (at < j) lo = mid + 1;
+        else hi = mid - 1;
       }
-      fill_cell<PopT>(s, cur, i, rhoL, rhoG, [&](long long j, Real &p, Real &r, Real &x, Real &y, Real &z) {
-        const int pos = j > i ? find(j) : -1;
-        if (pos >= 0) {
-          p = sOld[0][pos];
-          r = sOld[1][pos];
-          x = sOld[2][pos];
-          y = sOld[3][pos];
-          z = sOld[4][pos];
-        } else {
-          current(j, p, r, x, y, z);
+      if (i < 0 || dep >= 0 && sIdx[dep] < 0) dep = -1;
+      sDep[q][n] = (int8_t)dep;
+      if (dep >= 0) atomicOr(&sNeed[q], 1u << dep);
+    }
+#pragma unroll
+    for (int t = 0; t < FILL_GROUP / WARPS; t++) {
+      const int q = warp + t * WARPS, i = sIdx[q], j = i + dz * nxny + dy * s.nx + dx;
+      if (i < 0 || lane >= Q27) continue;
+      // (the tag from L2: other blocks of the same launch may have written it)
+      const bool fluid = __ldcg(s.tag + j) == TAG_FLUID;
+      const Real v[5] = {s.phi[cur][j], s.rho[cur][j], s.ux_at(cur, j), s.uy_at(cur, j), s.uz[cur][j]};
+      for (int c = 0; c < 5; c++) sVal[q][c][lane] = fluid ? v[c] : (Real)0;
+      if (lane == OWN) sVal[q][0][OWN] = v[0];
+      const unsigned fl = __ballot_sync((1u << Q27) - 1, fluid && lane != OWN);
+      if (lane == 0) sCnt[q] = __popc(fl);
+    }
+    __syncthreads();
+    const int q = threadIdx.x / 5, c = threadIdx.x % 5;
+    const int i = q < FILL_GROUP ? sIdx[q] : -1;
+    bool waiting = i >= 0;
+    while (__syncthreads_or(waiting)) {
+      const uint32_t done = sDone;
+      __syncthreads();
+      if (waiting && !(sNeed[q] & ~done)) {
+        double sum = 0;
+#pragma unroll
+        for (int n = 0; n < Q27; n++) {  // (a zero changes no sum)
+          if (n == OWN) continue;
+          const int dep = n < OWN ? sDep[q][n] : -1;
+          sum += (double)(dep >= 0 ? sVal[dep][c][OWN] : sVal[q][c][n]);
         }
-      });
-      sDone[q] = round;
+        const int cnt = sCnt[q];
+        const double mean = cnt > 0 ? sum / cnt : c == 0 ? (double)sVal[q][0][OWN] : c == 1 ? 1.0 : 0.0;
+        sMean[q][c] = mean;
+        sVal[q][c][OWN] = (Real)mean;
+        if (c == 0) s.phi[cur][i] = s.phi[1 - cur][i] = (Real)mean;  // phi and phiPrev
+        if (c == 1) s.rho[cur][i] = (Real)mean;
+        if (c == 2) s.set_ux(cur, i, (Real)mean);
+        if (c == 3) s.set_uy(cur, i, (Real)mean);
+        if (c == 4) s.uz[cur][i] = (Real)mean;
+        if (c == 0) atomicOr(&sDone, 1u << q);
+        waiting = false;
+      }
     }
-    if (!__syncthreads_or(waiting)) break;
+#pragma unroll 1
+    for (int e = warp; e < m; e += WARPS) {
+      const int at = sIdx[e];
+      if (at < 0 || lane >= Q27) continue;
+      const double p = sMean[e][0], r = sMean[e][1], vx = sMean[e][2], vy = sMean[e][3], vz = sMean[e][4];
+      const double rhoPhase = rhoG + p * (rhoL - rhoG);
+      const double u2 = vx * vx + vy * vy + vz * vz;
+      const double eu = ex * vx + ey * vy + ez * vz;
+      const double Qi = eu * (3.0 + 4.5 * eu) - 1.5 * u2;
+      const double fk = (double)w * (r + rhoPhase * Qi);
+      s.F[cur][pidx<27>(k, at)] = Codec<PopT>::enc((Real)fk, (Real)w);
+      if (k < Q7) {
+        const double hk = (double)w7 * p * (1 + 4.0 * eu);
+        s.H[cur][pidx<7>(k, at)] = Codec<PopT>::enc((Real)hk, (Real)w7 * (Real)p);
+      }
+    }
+    __syncthreads();
   }
 }
+
 // ---------------------------------------------------------------- SOLID cells
 // The step updates FLUID cells only; a SOLID cell keeps its values in both
 // halves.  It gets them into the half that the step writes when it turns SOLID
@@ -688,74 +655,77 @@ __device__ __forceinline__ void sets_body(const SmallArgs<PopT> &a, unsigned bid
     if (threadIdx.x == 0) *a.ticket = 0;
   }
 
-  // exclusive scan of the counts: each thread a run of chunks, then the block
-  const int per = (nch + SETS_THREADS - 1) / SETS_THREADS;
-  const int b0 = threadIdx.x * per, b1 = min(b0 + per, nch);
-  int2 sum = make_int2(0, 0);
-  for (int b = b0; b < b1; b++) {
-    const int2 v = __ldcg(a.counts + b);
-    sum.x += v.x;
-    sum.y += v.y;
-  }
-  int2 inc = sum;
-  for (int o = 1; o < 32; o <<= 1) {
-    const int fx = __shfl_up_sync(0xffffffffu, inc.x, o), fy = __shfl_up_sync(0xffffffffu, inc.y, o);
-    if (lane >= o) inc.x += fx, inc.y += fy;
-  }
-  if (lane == 31) sw[warp] = inc;
-  __syncthreads();
-  int2 run = make_int2(inc.x - sum.x, inc.y - sum.y), all = make_int2(0, 0);
-  for (int w = 0; w < SETS_THREADS / 32; w++) {
-    if (w < warp) run.x += sw[w].x, run.y += sw[w].y;
-    all.x += sw[w].x, all.y += sw[w].y;
+  // Per 256 chunks: exclusive scan of the counts, a queue of the chunks that
+  // hold any, then one warp per such chunk: lane l's two pairs of words (32
+  // cells each) in order, the next chunk's words on the way.  (Chunks given to
+  // the warps by place kept five of eight warps idle at 65 chunks: 28,000
+  // cycles where this takes 9,000.)
+  __shared__ int3 queue[SETS_THREADS];
+  __shared__ int queued;
+  int2 all = make_int2(0, 0);
+  for (int t0 = 0; t0 < nch; t0 += SETS_THREADS) {
+    const int mine = t0 + threadIdx.x;
+    const int2 cnt = mine < nch ? __ldcg(a.counts + mine) : make_int2(0, 0);
+    int2 inc = cnt;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int fx = __shfl_up_sync(0xffffffffu, inc.x, o), fy = __shfl_up_sync(0xffffffffu, inc.y, o);
+      if (lane >= o) inc.x += fx, inc.y += fy;
+    }
+    if (lane == 31) sw[warp] = inc;
+    if (threadIdx.x == 0) queued = 0;
+    __syncthreads();
+    int2 run = make_int2(all.x + inc.x - cnt.x, all.y + inc.y - cnt.y);
+    for (int w = 0; w < SETS_THREADS / 32; w++) {
+      const int2 v = sw[w];
+      if (w < warp) run.x += v.x, run.y += v.y;
+      all.x += v.x, all.y += v.y;
+    }
+    if (cnt.x | cnt.y) queue[atomicAdd(&queued, 1)] = make_int3(mine, run.x, run.y);
+    __syncthreads();
+    const int n = queued;
+    const uint4 *words = reinterpret_cast<const uint4 *>(a.bits) + lane;
+    uint4 next = make_uint4(0, 0, 0, 0);
+    if (warp < n) next = __ldcg(words + (long long)queue[warp].x * (SETS_WORDS / 2));
+#pragma unroll 1
+    for (int e = warp; e < n; e += SETS_THREADS / 32) {
+      const int3 at = queue[e];
+      const uint4 w = next;
+      if (e + SETS_THREADS / 32 < n)
+        next = __ldcg(words + (long long)queue[e + SETS_THREADS / 32].x * (SETS_WORDS / 2));
+      // fresh cells in the low half of a word, dead ones in the high half
+      const int m = __popc(w.x) + __popc(w.z) + ((__popc(w.y) + __popc(w.w)) << 16);
+      int pre = m;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, pre, o);
+        if (lane >= o) pre += x;
+      }
+      pre -= m;
+      int of = at.y + (pre & 0xffff), od = at.z + (pre >> 16);
+      unsigned l0 = (unsigned)at.x * COMPACT_CHUNK + 2 * lane * 32;
+#pragma unroll 1
+      for (int part = 0; part < 4; part++) {
+        const bool dead = part & 1;
+        unsigned bits = part == 0 ? w.x : part == 1 ? w.y : part == 2 ? w.z : w.w;
+        int *list = dead ? a.dead : a.fresh;
+        int pos = dead ? od : of;
+        for (; bits; bits &= bits - 1, pos++) {
+          const unsigned l = l0 + (part & 2) * 16 + (__ffs(bits) - 1), q = l / dx;
+          const int x = bx.lo[0] + (int)(l - q * dx), y = bx.lo[1] + (int)(q % dy), z = bx.lo[2] + (int)(q / dy);
+          if (pos < a.listCap) list[pos] = (z * s.ny + y) * s.nx + x;
+        }
+        if (dead) od = pos;
+        else of = pos;
+      }
+    }
+    __syncthreads();
   }
   if (threadIdx.x == 0) {
     a.totals[0] = all.x;
     a.totals[1] = all.y;
   }
-  if (all.x == 0 && all.y == 0) return;
-  // offsets of the chunks that hold any (y < 0 marks the others)
-  for (int b = b0; b < b1; b++) {
-    const int2 v = __ldcg(a.counts + b);
-    a.counts[b] = v.x | v.y ? run : make_int2(0, -1);
-    run.x += v.x;
-    run.y += v.y;
-  }
-  __syncthreads();
-  // one warp per such chunk: lane l's two words of 32 cells each, in order
-  for (int c0 = warp * 32; c0 < nch; c0 += SETS_THREADS) {
-    const int2 off = c0 + lane < nch ? a.counts[c0 + lane] : make_int2(0, -1);
-    unsigned busy = __ballot_sync(0xffffffffu, off.y >= 0);
-    for (; busy; busy &= busy - 1) {
-      const int src = __ffs(busy) - 1, c = c0 + src;
-      int of = __shfl_sync(0xffffffffu, off.x, src), od = __shfl_sync(0xffffffffu, off.y, src);
-      const uint4 w = __ldcg(reinterpret_cast<const uint4 *>(a.bits) + (long long)c * (SETS_WORDS / 2) + lane);
-      const int mf = __popc(w.x) + __popc(w.z), md = __popc(w.y) + __popc(w.w);
-      int pf = mf, pd = md;
-      for (int o = 1; o < 32; o <<= 1) {
-        const int x = __shfl_up_sync(0xffffffffu, pf, o), y = __shfl_up_sync(0xffffffffu, pd, o);
-        if (lane >= o) pf += x, pd += y;
-      }
-      of += pf - mf;
-      od += pd - md;
-      for (int h = 0; h < 2; h++) {
-        const unsigned l0 = (unsigned)c * COMPACT_CHUNK + (2 * lane + h) * 32;
-        auto put = [&](unsigned m, int *list, int &pos) {
-          for (; m; m &= m - 1, pos++) {
-            int x, y, z;
-            box_cell(bx, l0 + (__ffs(m) - 1), x, y, z);
-            if (pos < a.listCap) list[pos] = (z * s.ny + y) * s.nx + x;
-          }
-        };
-        put(h ? w.z : w.x, a.fresh, of);
-        put(h ? w.w : w.y, a.dead, od);
-      }
-    }
-  }
   if constexpr (FILL) {
     if (all.x == 0) return;
-    __syncthreads();
-    fresh_fill_body<PopT>(s, a.cur, a.fresh, min(all.x, a.listCap), a.rhoL, a.rhoG, a.zlo, a.zend, a.seqFill);
+    fresh_fill_body<PopT, SETS_THREADS>(s, a.cur, a.fresh, min(all.x, a.listCap), a.rhoL, a.rhoG, a.zlo, a.zend, a.seqFill);
   }
 }
 template <class PopT, bool RETAG, bool FILL>
