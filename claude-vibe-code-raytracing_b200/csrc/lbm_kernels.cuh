@@ -132,39 +132,6 @@ __global__ void k_seed_hydrostatic(Scene<PopT, typename Prec<PopT>::Real> s, int
   }
 }
 
-// =====================================================================================
-// Phase-by-phase kernels (FP32 and FP64 storage).  Reference semantics:
-// f = F[cur], f2 = F[1-cur]; h = H[cur], h2 = H[1-cur]; macros in place in
-// [cur]; phiPrev = phi[1-cur].
-
-// computePhiGradients (src/sim.js:176-199)
-template <class PopT>
-__global__ void k_gradients(Scene<PopT, typename Prec<PopT>::Real> s, int cur) {
-  using Real = typename Prec<PopT>::Real;
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= s.n) return;
-  const int nx = s.nx, ny = s.ny, nz = s.nz;
-  int x = (int)(i % nx);
-  long long t = i / nx;
-  int y = (int)(t % ny);
-  int z = (int)(t / ny);
-  int zm = z > 0 ? z - 1 : z, zp = z < nz - 1 ? z + 1 : z;
-  int ym = y > 0 ? y - 1 : y, yp = y < ny - 1 ? y + 1 : y;
-  int xm = x > 0 ? x - 1 : x, xp = x < nx - 1 ? x + 1 : x;
-  const Real *phi = s.phi[cur];
-  Real c = phi[i];
-  Real px = phi[cell_index(xp, y, z, nx, ny)];
-  Real mx = phi[cell_index(xm, y, z, nx, ny)];
-  Real py = phi[cell_index(x, yp, z, nx, ny)];
-  Real my = phi[cell_index(x, ym, z, nx, ny)];
-  Real pz = phi[cell_index(x, y, zp, nx, ny)];
-  Real mz = phi[cell_index(x, y, zm, nx, ny)];
-  s.gx[i] = (Real)0.5 * (px - mx);
-  s.gy[i] = (Real)0.5 * (py - my);
-  s.gz[i] = (Real)0.5 * (pz - mz);
-  s.lap[i] = px + mx + py + my + pz + mz - (Real)6 * c;
-}
-
 // retagCells over the whole grid (src/sim.js:214-244): tagPrev <- tag,
 // phiPrev <- phi, classification with FP64 contains, us = float(surfaceVelocity).
 template <class PopT>
@@ -175,10 +142,8 @@ __global__ void k_retag_full(Scene<PopT, typename Prec<PopT>::Real> s, int cur,
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= s.n) return;
   const int nx = s.nx, ny = s.ny, nz = s.nz;
-  int x = (int)(i % nx);
-  long long t = i / nx;
-  int y = (int)(t % ny);
-  int z = (int)(t / ny);
+  const unsigned t = (unsigned)i / (unsigned)nx;  // (n < 2^31 cells)
+  const int x = (int)((unsigned)i - t * (unsigned)nx), z = (int)(t / (unsigned)ny), y = (int)(t - (unsigned)z * (unsigned)ny);
   s.tagPrev[i] = s.tag[i];
   s.phi[1 - cur][i] = s.phi[cur][i];
   if (x == 0 || x == nx - 1 || y == 0 || y == ny - 1 || z == 0 || z == nz - 1) {
@@ -199,170 +164,6 @@ __global__ void k_retag_full(Scene<PopT, typename Prec<PopT>::Real> s, int cur,
     s.tag[i] = TAG_FLUID;
     s.usx[i] = s.usy[i] = s.usz[i] = (Real)0;
   }
-}
-
-// collidePhase (src/sim.js:324-364)
-template <class PopT>
-__global__ void k_collide_phase(Scene<PopT, typename Prec<PopT>::Real> s, int cur, StepConst k) {
-  using Real = typename Prec<PopT>::Real;
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= s.n || s.tag[i] != TAG_FLUID || !interior_cell(i, s.nx, s.ny, s.nz)) return;
-  const Real invTau = (Real)k.invTauPhi;
-  const Real sharpC = (Real)k.sharpC;
-  const Real sharpFac = (Real)4.0;
-  Real p = s.phi[cur][i];
-  Real uxi = s.ux_at(cur, i), uyi = s.uy_at(cur, i), uzi = s.uz[cur][i];
-  Real ggx = s.gx[i], ggy = s.gy[i], ggz = s.gz[i];
-  Real gmag = sqrt(ggx * ggx + ggy * ggy + ggz * ggz) + (Real)1e-12;
-  Real sharpen = sharpC * p * ((Real)1 - p);
-  Real Sx = sharpen * sharpFac * ggx / gmag;
-  Real Sy = sharpen * sharpFac * ggy / gmag;
-  Real Sz = sharpen * sharpFac * ggz / gmag;
-  const PopT *h = s.H[cur];
-  PopT *h2 = s.H[1 - cur];
-  for (int q = 0; q < Q7; q++) {
-    Real wk = (Real)w7_of(q);
-    Real ex = (Real)dcomp(q, 0), ey = (Real)dcomp(q, 1), ez = (Real)dcomp(q, 2);
-    Real eu = ex * uxi + ey * uyi + ez * uzi;
-    Real heq = wk * p * ((Real)1 + (Real)4 * eu);
-    Real Fk = wk * (ex * Sx + ey * Sy + ez * Sz);
-    Real hk = Codec<PopT>::dec(h[pidx<7>(q, i)], (Real)0);
-    h2[pidx<7>(q, i)] = Codec<PopT>::enc(hk - invTau * (hk - heq) + Fk, (Real)0);
-  }
-}
-
-// streamPhase (src/sim.js:376-397): pull with plain bounce-back.
-template <class PopT>
-__global__ void k_stream_phase(Scene<PopT, typename Prec<PopT>::Real> s, int cur) {
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= s.n || s.tag[i] != TAG_FLUID || !interior_cell(i, s.nx, s.ny, s.nz)) return;
-  const int nx = s.nx, ny = s.ny;
-  const PopT *h2 = s.H[1 - cur];
-  PopT *h = s.H[cur];
-  for (int q = 0; q < Q7; q++) {
-    long long src = i - (((long long)dcomp(q, 2) * ny + dcomp(q, 1)) * nx + dcomp(q, 0));
-    h[pidx<7>(q, i)] = s.tag[src] == TAG_FLUID ? h2[pidx<7>(q, src)] : h2[pidx<7>(opp_of(q), i)];
-  }
-}
-
-// collideHydro (src/sim.js:406-464)
-template <class PopT>
-__global__ void k_collide_hydro(Scene<PopT, typename Prec<PopT>::Real> s, int cur, StepConst k) {
-  using Real = typename Prec<PopT>::Real;
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= s.n || s.tag[i] != TAG_FLUID || !interior_cell(i, s.nx, s.ny, s.nz)) return;
-  const Real invTau = (Real)k.invTau;
-  const Real beta = (Real)k.beta, kappa = (Real)k.kappa, dRho = (Real)k.dRho;
-  const Real A = (Real)k.A, rhoG = (Real)k.rhoG, gravity = (Real)k.gravity;
-  Real sumF = s.rho[cur][i];
-  Real p = s.phi[cur][i];
-  Real rhoPhase = rhoG + p * dRho;
-  Real mu = (Real)4 * beta * p * (p - (Real)1) * ((Real)2 * p - (Real)1) - kappa * s.lap[i];
-  Real bx = s.bfx ? s.bfx[i] : (Real)0, by = s.bfy ? s.bfy[i] : (Real)0, bz = s.bfz ? s.bfz[i] : (Real)0;
-  Real fx = bx + mu * s.gx[i];
-  Real fy = by + mu * s.gy[i] + rhoPhase * gravity;
-  Real fz = bz + mu * s.gz[i];
-  Real uxe = s.ux_at(cur, i), uye = s.uy_at(cur, i), uze = s.uz[cur][i];
-  Real u2 = uxe * uxe + uye * uye + uze * uze;
-  Real negU2half = (Real)-1.5 * u2;
-  Real uF = uxe * fx + uye * fy + uze * fz;
-  const PopT *f = s.F[cur];
-  PopT *f2 = s.F[1 - cur];
-  for (int q = 0; q < Q27; q++) {
-    Real wk = (Real)w27_of(q);
-    Real ex = (Real)dcomp(q, 0), ey = (Real)dcomp(q, 1), ez = (Real)dcomp(q, 2);
-    Real eu = ex * uxe + ey * uye + ez * uze;
-    Real Qi = negU2half + eu * ((Real)3 + (Real)4.5 * eu);
-    Real feq = wk * (sumF + rhoPhase * Qi);
-    Real ekF = ex * fx + ey * fy + ez * fz;
-    Real Sk = A * wk * (ekF * ((Real)1 + (Real)3 * eu) - uF);
-    Real fk = Codec<PopT>::dec(f[pidx<27>(q, i)], (Real)0);
-    f2[pidx<27>(q, i)] = Codec<PopT>::enc(fk - invTau * (fk - feq) + Sk, (Real)0);
-  }
-}
-
-// streamHydroAndMacro (src/sim.js:484-582)
-template <class PopT>
-__global__ void k_stream_hydro_macro(Scene<PopT, typename Prec<PopT>::Real> s, int cur,
-                                     StepConst kc, const SolidSet *__restrict__ ssp) {
-  const SolidSet &ss = *ssp;
-  using Real = typename Prec<PopT>::Real;
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= s.n || s.tag[i] != TAG_FLUID || !interior_cell(i, s.nx, s.ny, s.nz)) return;
-  const int nx = s.nx, ny = s.ny;
-  int x = (int)(i % nx);
-  long long t = i / nx;
-  int y = (int)(t % ny);
-  int z = (int)(t / ny);
-  const Real beta = (Real)kc.beta, kappa = (Real)kc.kappa, dRho = (Real)kc.dRho;
-  const Real rhoG = (Real)kc.rhoG, gravity = (Real)kc.gravity;
-  const PopT *f2 = s.F[1 - cur];
-  PopT *f = s.F[cur];
-  Real rhoPhaseOld = rhoG + s.phi[cur][i] * dRho;
-  Real pSumF = 0, mx = 0, my = 0, mz = 0;
-  double acc[6] = {0, 0, 0, 0, 0, 0};
-  int owner = -1;
-  for (int q = 0; q < Q27; q++) {
-    const int ex = dcomp(q, 0), ey = dcomp(q, 1), ez = dcomp(q, 2);
-    long long src = i - (((long long)ez * ny + ey) * nx + ex);
-    uint8_t sTag = s.tag[src];
-    Real fk;
-    if (sTag == TAG_FLUID) {
-      fk = Codec<PopT>::dec(f2[pidx<27>(q, src)], (Real)0);
-    } else {
-      Real fopp = Codec<PopT>::dec(f2[pidx<27>(opp_of(q), i)], (Real)0);
-      Real corr = 0;
-      if (sTag == TAG_SOLID) {
-        Real eu = (Real)ex * s.usx[src] + (Real)ey * s.usy[src] + (Real)ez * s.usz[src];
-        corr = (Real)2 * (Real)w27_of(q) * rhoPhaseOld * eu * (Real)3;
-      }
-      fk = fopp + corr;
-      if (sTag == TAG_SOLID && ss.nsph > 0) {
-        int sx = x - ex, sy = y - ey, sz = z - ez;
-        int b = owner_of<LBM_MAX_SPHERES>(ss.sph, ss.nsph, sx, sy, sz);
-        if (b >= 0) {
-          if (b != owner) {
-            flush_impulse(ss, owner, x, y, z, acc);
-            owner = b;
-          }
-          double m = __dadd_rn((double)fopp, (double)fk);
-          impulse_terms(ss.sph[b], sx, sy, sz, -m * ex, -m * ey, -m * ez, acc);
-        }
-      }
-    }
-    f[pidx<27>(q, i)] = Codec<PopT>::enc(fk, (Real)0);
-    pSumF += fk;
-    mx += (Real)ex * fk;
-    my += (Real)ey * fk;
-    mz += (Real)ez * fk;
-  }
-  flush_impulse(ss, owner, x, y, z, acc);
-  s.rho[cur][i] = pSumF > (Real)0.01 ? pSumF : (Real)0.01;
-  Real phiSum = 0;
-  for (int q = 0; q < Q7; q++) phiSum += Codec<PopT>::dec(s.H[cur][pidx<7>(q, i)], (Real)0);
-  Real p = phiSum < (Real)0 ? (Real)0 : phiSum > (Real)1 ? (Real)1 : phiSum;
-  s.phi[cur][i] = p;
-  Real rhoPhaseNew = rhoG + p * dRho;
-  Real mu = (Real)4 * beta * p * (p - (Real)1) * ((Real)2 * p - (Real)1) - kappa * s.lap[i];
-  Real bx = s.bfx ? s.bfx[i] : (Real)0, by = s.bfy ? s.bfy[i] : (Real)0, bz = s.bfz ? s.bfz[i] : (Real)0;
-  Real fx = bx + mu * s.gx[i];
-  Real fy = by + mu * s.gy[i] + rhoPhaseNew * gravity;
-  Real fz = bz + mu * s.gz[i];
-  Real invRho = (Real)1 / rhoPhaseNew;
-  Real uxn = (mx + (Real)0.5 * fx) * invRho;
-  Real uyn = (my + (Real)0.5 * fy) * invRho;
-  Real uzn = (mz + (Real)0.5 * fz) * invRho;
-  Real u2 = uxn * uxn + uyn * uyn + uzn * uzn;
-  const Real UMAX = (Real)0.2, UMAX2 = (Real)(0.2 * 0.2);
-  if (u2 > UMAX2) {
-    Real sc = UMAX / sqrt(u2);
-    uxn *= sc;
-    uyn *= sc;
-    uzn *= sc;
-  }
-  s.set_ux(cur, i, uxn);
-  s.set_uy(cur, i, uyn);
-  s.uz[cur][i] = uzn;
 }
 
 // =====================================================================================

@@ -9,6 +9,7 @@
 
 #include "lbm_fused_pipe.cuh"
 #include "lbm_kernels.cuh"
+#include "lbm_phases.cuh"
 #include "lbm_shell.cuh"
 #include "lbm_sphere.cuh"
 #include "lbm_state.h"
@@ -111,7 +112,8 @@ class Ops final : public OpsBase {
 
   size_t pop_bytes() const override { return sizeof(PopT); }
   size_t macro_bytes() const override { return sizeof(Real); }
-  bool phases_supported() const override { return !Codec<PopT>::offset; }
+  static constexpr bool PHASES = !Codec<PopT>::offset;
+  bool phases_supported() const override { return PHASES; }
 
   static SceneT scene(lbm_sim *h) {
     SceneT s;
@@ -155,8 +157,10 @@ class Ops final : public OpsBase {
     h->launches++;
   }
   void gradients(lbm_sim *h) override {
-    k_gradients<PopT><<<nblocks(h->n, 256), 256, 0, h->stream>>>(scene(h), h->cur);
-    h->launches++;
+    if constexpr (PHASES) {
+      k_gradients<PopT><<<nblocks(h->n, PHASE_THREADS), PHASE_THREADS, 0, h->stream>>>(scene(h), h->cur);
+      h->launches++;
+    }
   }
   void retag_full(lbm_sim *h) override {
     k_retag_full<PopT><<<nblocks(h->n, 256), 256, 0, h->stream>>>(scene(h), h->cur, &h->plan()->ss);
@@ -178,23 +182,31 @@ class Ops final : public OpsBase {
     h->launches++;
   }
   void collide_phase(lbm_sim *h) override {
-    k_collide_phase<PopT><<<nblocks(h->n, 256), 256, 0, h->stream>>>(scene(h), h->cur,
-                                                                       make_const(h->params));
-    h->launches++;
+    if constexpr (PHASES) {
+      k_collide_phase<PopT><<<nblocks(h->n, PHASE_THREADS), PHASE_THREADS, 0, h->stream>>>(
+          scene(h), h->cur, make_const(h->params));
+      h->launches++;
+    }
   }
   void stream_phase(lbm_sim *h) override {
-    k_stream_phase<PopT><<<nblocks(h->n, 256), 256, 0, h->stream>>>(scene(h), h->cur);
-    h->launches++;
+    if constexpr (PHASES) {
+      k_stream_phase<PopT><<<nblocks(h->n, PHASE_THREADS), PHASE_THREADS, 0, h->stream>>>(scene(h), h->cur);
+      h->launches++;
+    }
   }
   void collide_hydro(lbm_sim *h) override {
-    k_collide_hydro<PopT><<<nblocks(h->n, 256), 256, 0, h->stream>>>(scene(h), h->cur,
-                                                                       make_const(h->params));
-    h->launches++;
+    if constexpr (PHASES) {
+      k_collide_hydro<PopT><<<nblocks(h->n, PHASE_THREADS), PHASE_THREADS, 0, h->stream>>>(
+          scene(h), h->cur, make_const(h->params));
+      h->launches++;
+    }
   }
   void stream_hydro_macro(lbm_sim *h) override {
-    k_stream_hydro_macro<PopT><<<nblocks(h->n, 256), 256, 0, h->stream>>>(
-        scene(h), h->cur, make_const(h->params), &h->plan()->ss);
-    h->launches++;
+    if constexpr (PHASES) {
+      k_stream_hydro_macro<PopT><<<nblocks(h->n, PHASE_THREADS), PHASE_THREADS, 0, h->stream>>>(
+          scene(h), h->cur, make_const(h->params), &h->plan()->ss);
+      h->launches++;
+    }
   }
   // the sparse kernels' arguments for the step that reads half cur
   static SmallArgs<PopT> small(lbm_sim *h, int cur) {
