@@ -96,9 +96,13 @@ struct FusedSmem {
 };
 
 // CTAs per SM the register budget is sized for
+// (FP64: as many as its ring leaves room for; sized for three, the kernel kept
+// 96 registers, spilled 680 B a thread and took 267 us a step at 96x80x72,
+// now 224)
 template <class PopT, int TY>
 struct FusedOcc {
-  static constexpr int blocks = TY >= 8 ? 2 : (TY >= 4 ? 3 : 5);
+  static constexpr int fit = (int)((227 * 1024) / (FusedSmem<PopT, TY>::bytes + 1024));
+  static constexpr int blocks = sizeof(PopT) == 8 ? fit : TY >= 8 ? 2 : (TY >= 4 ? 3 : 5);
 };
 
 // ---------------------------------------------------------------- bulk copies
