@@ -10,6 +10,7 @@
 #include <string>
 #include <vector>
 
+#include "lbm_hostcopy.h"
 #include "lbm_kernels.cuh"
 #include "lbm_mesh.cuh"
 #include "lbm_render.h"
@@ -102,6 +103,12 @@ cudaError_t copy_async(lbm_sim *h, void *dst, const void *src, size_t bytes, cud
   if (kind == cudaMemcpyHostToDevice) h->h2dBytes += bytes;
   if (kind == cudaMemcpyDeviceToHost) h->d2hBytes += bytes;
   return cudaMemcpyAsync(dst, src, bytes, kind, s);
+}
+
+// A result of the handle's stream into host memory, complete on return.
+cudaError_t copy_out(lbm_sim *h, void *dst, const void *src, size_t bytes) {
+  h->d2hBytes += bytes;
+  return copy_to_host(dst, src, bytes, h->device, h->stream);
 }
 
 int ensure_staging(lbm_sim *h, size_t bytes) {
@@ -491,16 +498,15 @@ int put_scalar(lbm_sim *h, void *dst, const float *host) {
 int get_scalar(lbm_sim *h, const void *src, float *host) {
   size_t n = (size_t)h->n;
   if (h->ops->macro_bytes() == 4) {
-    CK(copy_async(h, host, src, n * 4, cudaMemcpyDeviceToHost, h->stream));
+    CK(copy_out(h, host, src, n * 4));
   } else {
     int rc = ensure_staging(h, n * 4);
     if (rc) return rc;
     k_real_d_to_f32<<<nblocks(n, 256), 256, 0, h->stream>>>((float *)h->staging, (const double *)src, n);
     h->launches++;
     CKL("convert");
-    CK(copy_async(h, host, h->staging, n * 4, cudaMemcpyDeviceToHost, h->stream));
+    CK(copy_out(h, host, h->staging, n * 4));
   }
-  CK(cudaStreamSynchronize(h->stream));
   return LBM_OK;
 }
 
@@ -508,16 +514,15 @@ int get_scalar(lbm_sim *h, const void *src, float *host) {
 int get_scalar64(lbm_sim *h, const void *src, double *host) {
   size_t n = (size_t)h->n;
   if (h->ops->macro_bytes() == 8) {
-    CK(copy_async(h, host, src, n * 8, cudaMemcpyDeviceToHost, h->stream));
+    CK(copy_out(h, host, src, n * 8));
   } else {
     int rc = ensure_staging(h, n * 8);
     if (rc) return rc;
     k_f32_to_real_d<<<nblocks(n, 256), 256, 0, h->stream>>>((double *)h->staging, (const float *)src, n);
     h->launches++;
     CKL("convert");
-    CK(copy_async(h, host, h->staging, n * 8, cudaMemcpyDeviceToHost, h->stream));
+    CK(copy_out(h, host, h->staging, n * 8));
   }
-  CK(cudaStreamSynchronize(h->stream));
   return LBM_OK;
 }
 
@@ -619,7 +624,8 @@ int coupled_frame(lbm_sim *h, uint8_t *dst, bool fused = false) {
   if (fused) h->ops->pack_end_planes(h, (uint8_t *)h->staging);
   else h->ops->pack(h, (uint8_t *)h->staging);
   CKL("packVolume");
-  CK(copy_async(h, dst, h->staging, (size_t)h->n * 2, cudaMemcpyDeviceToHost, h->stream));
+  if (fused && pageable(dst)) CK(copy_out(h, dst, h->staging, (size_t)h->n * 2));
+  else CK(copy_async(h, dst, h->staging, (size_t)h->n * 2, cudaMemcpyDeviceToHost, h->stream));
   return LBM_OK;
 }
 
@@ -785,6 +791,7 @@ int lbm_create(int nx, int ny, int nz, int storage, int device, lbm_sim **out) {
   // A fresh Sim has every cell FLUID (zeroed Uint8Array); the first retag
   // covers the whole grid so the walls get their tags.
   h->fullRetagSteps = 2;
+  host_ring().attach();
   *out = h;
   return LBM_OK;
 }
@@ -795,6 +802,7 @@ int lbm_destroy(lbm_sim *h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   free_all(h);
   delete h;
+  host_ring().detach();
   return LBM_OK;
 }
 
@@ -851,9 +859,7 @@ static int pops_transfer(lbm_sim *h, int field, const float *up, float *down) {
     } else {
       h->ops->download_pops(h, isH, second ? 2 : 1, (float *)h->staging, c0, cells);
       CKL("download populations");
-      CK(copy_async(h, down + c0 * Q, h->staging, cells * Q * sizeof(float), cudaMemcpyDeviceToHost,
-                         h->stream));
-      CK(cudaStreamSynchronize(h->stream));
+      CK(copy_out(h, down + c0 * Q, h->staging, cells * Q * sizeof(float)));
     }
   }
   return LBM_OK;
@@ -958,9 +964,7 @@ int lbm_download_field(lbm_sim *h, int field, void *host, size_t count) {
       return pops_transfer(h, field, nullptr, dst);
     case LBM_FIELD_TAG:
     case LBM_FIELD_TAG_PREV:
-      CK(copy_async(h, host, field == LBM_FIELD_TAG ? h->tag : h->tagPrev, n, cudaMemcpyDeviceToHost,
-                         h->stream));
-      CK(cudaStreamSynchronize(h->stream));
+      CK(copy_out(h, host, field == LBM_FIELD_TAG ? h->tag : h->tagPrev, n));
       return LBM_OK;
     case LBM_FIELD_PHI_PREV:
       return get_scalar(h, h->mac[1 - h->cur][0], dst);
@@ -1009,9 +1013,7 @@ int lbm_download_field_f64(lbm_sim *h, int field, double *host, size_t count) {
       long long cells = std::min(chunk, h->n - c0);
       h->ops->download_pops64(h, isH, second ? 2 : 1, (double *)h->staging, c0, cells);
       CKL("download populations");
-      CK(copy_async(h, host + c0 * Q, h->staging, cells * Q * sizeof(double), cudaMemcpyDeviceToHost,
-                    h->stream));
-      CK(cudaStreamSynchronize(h->stream));
+      CK(copy_out(h, host + c0 * Q, h->staging, cells * Q * sizeof(double)));
     }
     return LBM_OK;
   }
@@ -1543,8 +1545,7 @@ int lbm_pack_volume(lbm_sim *h, uint8_t *host_out) {
   if (rc) return rc;
   h->ops->pack(h, (uint8_t *)h->staging);
   CKL("packVolume");
-  CK(copy_async(h, host_out, h->staging, (size_t)h->n * 2, cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
+  CK(copy_out(h, host_out, h->staging, (size_t)h->n * 2));
   return LBM_OK;
 }
 
@@ -2141,10 +2142,20 @@ int lbm_batch_run(lbm_batch *b, lbm_sphere *const *spheres, const int *nspheres,
       BCK(cudaStreamWaitEvent(b->origin, b->joins[s], 0));
     }
     BCK(cudaStreamSynchronize(b->origin));
-    for (int s = 0; s < n; s++) {
-      const size_t one = 2 * (size_t)b->sims[s]->n;
-      memcpy(frames[s] + (size_t)idx * one, b->pinned + slot[s], one);
-    }
+    // out of the page-locked slots, the scenes' pieces side by side
+    std::atomic<size_t> next{0};
+    auto work = [&]() {
+      size_t piece = next++, first = 0;  // pieces are claimed in the scenes' order
+      for (int s = 0; s < n; s++) {
+        const size_t one = 2 * (size_t)b->sims[s]->n, pieces = (one + HOSTCOPY_PIECE - 1) / HOSTCOPY_PIECE;
+        for (; piece < first + pieces; piece = next++) {
+          const size_t o = (piece - first) * HOSTCOPY_PIECE;
+          memcpy(frames[s] + (size_t)idx * one + o, b->pinned + slot[s] + o, std::min(HOSTCOPY_PIECE, one - o));
+        }
+        first += pieces;
+      }
+    };
+    hostcopy_run(hostcopy_threads(slot[n]), work);
     return LBM_OK;
   };
 
