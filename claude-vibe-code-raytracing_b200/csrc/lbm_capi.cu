@@ -339,7 +339,7 @@ void launch_fused(lbm_sim *h) {
 // before a fused step: SOLID cells the same in both halves
 int ready_solid(lbm_sim *h) {
   if (!h->carrySolid) return LBM_OK;
-  h->ops->carry_solid(h);
+  h->ops->carry_solid(h, 0, h->n);
   CKL("SOLID cells");
   h->carrySolid = false;
   return LBM_OK;
@@ -1814,9 +1814,13 @@ int lbm_slab_copy_planes(lbm_sim *dst, int dst_plane, const lbm_sim *src, int sr
     CK(copy((char *)dst->mac[dst->cur][a] + dc * mb, (const char *)src->mac[src->cur][a] + sc * mb,
             (size_t)cells * mb));
   CK(copy(dst->tag + dc, src->tag + sc, (size_t)cells));
+  // the copies are of the current half alone.  (Carried here over these planes:
+  // left to the next step, which does not know them, it swept the whole slab,
+  // in every step of a scene of slabs.)
+  dst->ops->carry_solid(dst, dc, dc + cells);
+  CKL("SOLID cells of the copied planes");
   CK(cudaStreamSynchronize(dst->stream));
   dst->listsValid = false;
-  dst->carrySolid = true;
   return LBM_OK;
 }
 

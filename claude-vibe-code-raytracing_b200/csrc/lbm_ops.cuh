@@ -228,8 +228,8 @@ class Ops final : public OpsBase {
     a.rhoG = h->params.rhoG;
     return a;
   }
-  void carry_solid(lbm_sim *h) override {
-    k_carry_solid<PopT><<<std::min(nblocks(h->n, 256), 148u * 8u), 256, 0, h->stream>>>(scene(h), h->cur);
+  void carry_solid(lbm_sim *h, long long c0, long long c1) override {
+    k_carry_solid<PopT><<<std::min(nblocks(c1 - c0, 256), 148u * 8u), 256, 0, h->stream>>>(scene(h), h->cur, c0, c1);
     h->launches++;
   }
   void sets(lbm_sim *h, long long maxChunks, bool retag, bool fill) override {

@@ -104,7 +104,8 @@ class OpsBase {
   virtual void stream_phase(lbm_sim *h) = 0;
   virtual void collide_hydro(lbm_sim *h) = 0;
   virtual void stream_hydro_macro(lbm_sim *h) = 0;
-  virtual void carry_solid(lbm_sim *h) = 0;  // every SOLID cell: current half -> the other
+  // the SOLID cells of [c0, c1): current half -> the other
+  virtual void carry_solid(lbm_sim *h, long long c0, long long c1) = 0;
   // retag on the plan's box (retag), fresh / dead lists, fresh fill (fill)
   virtual void sets(lbm_sim *h, long long maxChunks, bool retag, bool fill) = 0;
   virtual void absorb_dead(lbm_sim *h, double *d_out) = 0;
@@ -253,7 +254,7 @@ struct lbm_sim {
   int stepBegunNs = -1;
   bool planOfStep = false;  // the device plan is the begun step's
   // a SOLID cell may differ between the halves (a field write, a phase-by-phase
-  // call, copied planes): carried over the whole grid before the next fused step
+  // call): carried over the whole grid before the next fused step
   bool carrySolid = false;
   int fullRetagSteps = 0;
   int nsphLast = 0;

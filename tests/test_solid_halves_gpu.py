@@ -1,0 +1,58 @@
+"""SOLID cells through the calls that touch one half, or their tags, between
+steps: nothing is computed for a SOLID cell, so it holds one value in both
+halves whatever number of steps follows."""
+import numpy as np
+import pytest
+
+import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    import torch
+    assert torch.cuda.is_available(), "GPU tests need a CUDA device"
+    import b200lbm
+    return b200lbm
+
+
+DIMS = (32, 17, 26)  # (nx * ny divisible by 8: plane copies)
+
+
+def _tank(gpu, storage="f32", level=8, dims=DIMS):
+    sim = gpu.Sim(*dims, storage=storage)
+    scenes._params(sim, 0.8, 0.7, 0.008, 0.0015)
+    sim.initFlat(level)
+    sol = gpu.RigidSphere(*dims, cx=dims[0] / 2 + 0.3, cy=dims[1] / 2 + 0.1, cz=dims[2] / 2 - 0.4, r=4.2, density=2.0)
+    return sim, sol
+
+
+def _cells(sim, k):
+    return np.array(getattr(sim, k)).reshape(sim.n, -1)
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16", "f64"])
+def test_copied_planes_hold_their_solid_cells_in_both_halves(gpu, storage):
+    """lbm_slab_copy_planes copies the current half; the SOLID cells of those
+    planes, and no others, are the same in the other half when it returns."""
+    (src, sol), (dst, _) = _tank(gpu, storage, 8), _tank(gpu, storage, 12)
+    for _ in range(2):
+        src.step(sol)
+        dst.step(sol)
+    was = {k: _cells(dst, k) for k in ("f", "f2", "h2")}
+    plane, nxny = 12, DIMS[0] * DIMS[1]
+    gpu._capi.check(dst.handle, gpu._capi.lib().lbm_slab_copy_planes(dst.handle, plane, src.handle, plane, 2))
+    dst._moved()
+    z = np.arange(dst.n) // nxny
+    solid = np.asarray(dst.tag) == 1
+    copied = solid & (z >= plane) & (z < plane + 2)
+    assert copied.sum() > 60
+    assert not np.array_equal(_cells(src, "f")[copied], was["f"][copied])
+    for k, k2 in (("f", "f2"), ("h", "h2")):
+        assert np.array_equal(_cells(dst, k)[copied], _cells(src, k)[copied]), k
+        assert np.array_equal(_cells(dst, k2)[copied], _cells(src, k)[copied]), k2
+    for k in ("f2", "h2"):
+        assert np.array_equal(_cells(dst, k)[~copied], was[k][~copied]), k
+    src.close()
+    dst.close()
