@@ -1367,6 +1367,7 @@ int lbm_step_end(lbm_sim *h, const lbm_sphere *sp, int ns, lbm_impulse *out) {
     if ((rc = lbm_collide_hydro(h))) return rc;
     return lbm_stream_hydro_and_macro(h, sp, ns, out);
   }
+  if ((rc = ready_solid(h))) return rc;  // (fields may have been written since the step began)
   if (!h->planOfStep) {  // another call has put its own plan in place since the step began
     if ((rc = set_solids(h, sp, ns, true))) return rc;
     set_box(h, h->lastRetagBox);

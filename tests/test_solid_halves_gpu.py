@@ -56,3 +56,29 @@ def test_copied_planes_hold_their_solid_cells_in_both_halves(gpu, storage):
         assert np.array_equal(_cells(dst, k)[~copied], was[k][~copied]), k
     src.close()
     dst.close()
+
+
+FIELDS = ("f", "h", "phi", "rho", "ux", "uy", "uz")
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16", "f64"])
+@pytest.mark.parametrize("write", ["tag", "f2"])
+def test_a_write_inside_a_split_step(gpu, storage, write):
+    """Cells written SOLID, and SOLID cells whose other half was written,
+    between step_begin and step_end keep their values through the step."""
+    sim, sol = _tank(gpu, storage)
+    for _ in range(4):
+        sim.step(sol)
+    sim.step_begin(sol)
+    if write == "tag":
+        for at in ((4, 12, 5), (5, 12, 5), (9, 13, 20), (16, 13, 12)):
+            sim.tag[sim.idx(*at)] = 1
+    else:
+        sim.f2[:] = np.float32(0.25)
+        sim.h2[:] = np.float32(0.125)
+    solid = np.asarray(sim.tag) == 1
+    want = {k: _cells(sim, k)[solid] for k in FIELDS}
+    sim.step_end(sol)
+    for k in FIELDS:
+        assert np.array_equal(_cells(sim, k)[solid], want[k]), k
+    sim.close()
