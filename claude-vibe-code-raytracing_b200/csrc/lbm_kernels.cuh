@@ -428,7 +428,8 @@ __device__ __forceinline__ void sets_body(const SmallArgs<PopT> &a, unsigned bid
         }
         isF = t[j] == TAG_FLUID && p[j] == TAG_SOLID;
         isD = t[j] == TAG_SOLID && p[j] == TAG_FLUID;
-        if (RETAG && isD) carry_cell<PopT>(s, a.cur, cell[j]);
+        // (also a cell that a written tag made WALL, which is no dead cell)
+        if (RETAG && t[j] == TAG_SOLID && p[j] != TAG_SOLID) carry_cell<PopT>(s, a.cur, cell[j]);
       }
       const unsigned bf = __ballot_sync(0xffffffffu, isF), bd = __ballot_sync(0xffffffffu, isD);
       if (lane == 0)

@@ -62,6 +62,35 @@ FIELDS = ("f", "h", "phi", "rho", "ux", "uy", "uz")
 
 
 @pytest.mark.parametrize("storage", ["f32", "f16", "f64"])
+@pytest.mark.parametrize("how", ["step", "run_coupled", "batch"])
+def test_walls_that_turn_solid(gpu, storage, how):
+    """Interior cells written WALL that the sphere then covers."""
+    sim, sol = _tank(gpu, storage)
+    away = gpu.RigidSphere(*DIMS, cx=5.2, cy=5.1, cz=5.3, r=1.4, density=2.0)
+    for _ in range(3):
+        sim.step(away)
+    tag = np.array(sim.tag).reshape(DIMS[::-1])
+    tag[8:17, 6:13, 12:21] = 2
+    sim.tag[:] = tag.ravel()
+    before = {k: _cells(sim, k) for k in FIELDS}
+    sol.vx = sol.vy = sol.vz = 0.0
+    for t in range(3):
+        if how == "step":
+            sim.step(sol)
+        elif how == "run_coupled":
+            sim.run_coupled(sol, 1)
+        else:
+            with gpu.Batch([(sim, sol)]) as batch:
+                batch.run(1)
+        now = np.asarray(sim.tag) == 1
+        solid = now & (tag.ravel() == 2)  # (the sphere moves less than a cell)
+        assert solid.sum() > 100
+        for k in FIELDS:
+            assert np.array_equal(_cells(sim, k)[solid], before[k][solid]), (t, k)
+    sim.close()
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16", "f64"])
 @pytest.mark.parametrize("write", ["tag", "f2"])
 def test_a_write_inside_a_split_step(gpu, storage, write):
     """Cells written SOLID, and SOLID cells whose other half was written,
