@@ -317,8 +317,12 @@ int default_zchunk(lbm_sim *const *sims, int n) {
   });
 }
 
-// The fused step kernel, bracketed by CUDA events when timing is on.
-void launch_fused(lbm_sim *h) {
+// The fused step kernel, bracketed by CUDA events when timing is on.  anyTag:
+// the tags may not be the retag's, and in the plain form, which takes the tags
+// of the domain's faces as they are (the others know those cells for walls).
+void launch_fused(lbm_sim *h, bool anyTag = false) {
+  FusedCfg cfg = h->cfg;
+  if (anyTag) cfg.ty = 4;
   if (h->timing) {
     if (h->evUsed == h->evStart.size()) {
       cudaEvent_t a, b;
@@ -328,11 +332,11 @@ void launch_fused(lbm_sim *h) {
       h->evStop.push_back(b);
     }
     cudaEventRecord(h->evStart[h->evUsed], h->stream);
-    h->ops->fused_step(h, h->cfg);
+    h->ops->fused_step(h, cfg);
     cudaEventRecord(h->evStop[h->evUsed], h->stream);
     h->evUsed++;
   } else {
-    h->ops->fused_step(h, h->cfg);
+    h->ops->fused_step(h, cfg);
   }
 }
 
@@ -589,6 +593,7 @@ int coupled_prepare(lbm_sim *h, const lbm_sphere *sp, int ns, bool frames, Coupl
   c.maxChunks = (c.maxU + COMPACT_CHUNK - 1) / COMPACT_CHUNK;
   c.redChunks = (int)((c.slotCells + RED_CHUNK - 1) / RED_CHUNK);
   c.tail = true;
+  h->tagsOfStep = false;  // (of a step that was begun and not ended)
   if ((rc = ready_solid(h))) return rc;
   if ((rc = ensure_work(h, std::max(1LL, (long long)ns * c.slotCells * 6),
                         (long long)std::max(ns, 1) * c.redChunks * 6)))
@@ -886,6 +891,7 @@ int lbm_upload_field(lbm_sim *h, int field, const void *host, size_t count) {
       CK(cudaStreamSynchronize(h->stream));
       h->fullRetagSteps = 2;
       h->listsValid = false;
+      h->tagsOfStep = false;
       return LBM_OK;
     case LBM_FIELD_PHI_PREV:
       // phiPrev is overwritten from phi by the next retagCells before anything
@@ -1049,6 +1055,7 @@ int lbm_init_flat(lbm_sim *h, double waterlineY) {
   h->boxLast = h->boxLastLast = Box{{1, 1, 1}, {0, 0, 0}};
   h->fullRetagSteps = 0;
   h->listsValid = false;
+  h->tagsOfStep = false;
   return LBM_OK;
 }
 
@@ -1064,6 +1071,7 @@ int lbm_init_profile(lbm_sim *h, const double *phi_col, int ny) {
   h->boxLast = h->boxLastLast = Box{{1, 1, 1}, {0, 0, 0}};
   h->fullRetagSteps = 0;
   h->listsValid = false;
+  h->tagsOfStep = false;
   return LBM_OK;
 }
 
@@ -1098,6 +1106,7 @@ int lbm_retag_cells(lbm_sim *h, const lbm_sphere *sp, int ns) {
   h->lastRetagBox = interior(h);
   h->fullRetagSteps = h->fullRetagSteps > 0 ? h->fullRetagSteps - 1 : 0;
   h->listsValid = false;
+  h->tagsOfStep = false;
   return LBM_OK;
 }
 
@@ -1120,6 +1129,7 @@ int lbm_retag_cells_mask(lbm_sim *h, const uint8_t *solid_mask, const float *sur
   h->fullRetagSteps = 2;
   h->lastRetagBox = interior(h);
   h->listsValid = false;
+  h->tagsOfStep = false;
   return LBM_OK;
 }
 
@@ -1200,6 +1210,7 @@ int lbm_retag_cells_mesh(lbm_sim *h, const double *tri, int ntri, const lbm_rigi
   h->fullRetagSteps = 2;
   h->lastRetagBox = interior(h);
   h->listsValid = false;
+  h->tagsOfStep = false;
   return LBM_OK;
 }
 
@@ -1347,6 +1358,7 @@ int lbm_step_begin(lbm_sim *h, const lbm_sphere *sp, int ns) {
   h->lastRetagBox = U;
   if ((rc = launch_sets(h, h->hPlan.nchunks, true, true))) return rc;
   h->planOfStep = true;
+  h->tagsOfStep = true;
   h->stepNow = now;
   h->stepBegunNs = ns;
   return LBM_OK;
@@ -1368,29 +1380,37 @@ int lbm_step_end(lbm_sim *h, const lbm_sphere *sp, int ns, lbm_impulse *out) {
     return lbm_stream_hydro_and_macro(h, sp, ns, out);
   }
   if ((rc = ready_solid(h))) return rc;  // (fields may have been written since the step began)
-  if (!h->planOfStep) {  // another call has put its own plan in place since the step began
+  const bool newPlan = !h->planOfStep;
+  if (newPlan) {  // another call has put its own plan in place since the step began
     if ((rc = set_solids(h, sp, ns, true))) return rc;
     set_box(h, h->lastRetagBox);
     if ((rc = upload_plan(h))) return rc;
   }
-  launch_fused(h);
+  const bool anyTag = !h->tagsOfStep || newPlan;
+  launch_fused(h, anyTag);
   CKL("fused step");
   if ((rc = flush_frame_copy(h))) return rc;
   if (ns > 0) {
     // the shell launch also computes absorbDeadCells, which follows every step
     // (src/worker.js:96-100) and reads only this step's dead list and values
     // that the step leaves alone: fetched with the step's impulses below, so
-    // lbm_absorb_dead_cells needs no launch and no wait of its own
+    // lbm_absorb_dead_cells needs no launch and no wait of its own (unless the
+    // tags have been written since: then it makes the list anew)
     StepCtx c;
     c.ns = ns;
     c.redChunks = h->partialsChunks;
+    c.anyTag = anyTag;
     h->ops->shell(h, c);
     CKL("shells");
+  }
+  if (anyTag) {
+    h->ops->finish_unowned(h);
+    CKL("cells next to SOLID cells of no sphere");
   }
   h->cur = 1 - h->cur;
   shift_boxes(h, h->stepNow);
   h->deadAhead.valid = false;
-  if (ns > 0 && out) {
+  if (ns > 0 && out && !anyTag) {
     CK(copy_async(h, h->hOut + LBM_MAX_SPHERES * 6, h->dOut + LBM_MAX_SPHERES * 6, (size_t)ns * 6 * sizeof(double),
                   cudaMemcpyDeviceToHost, h->stream));
     if ((rc = fetch_out(h, h->dOut, ns, out))) return rc;
@@ -1822,6 +1842,7 @@ int lbm_slab_copy_planes(lbm_sim *dst, int dst_plane, const lbm_sim *src, int sr
   CKL("SOLID cells of the copied planes");
   CK(cudaStreamSynchronize(dst->stream));
   dst->listsValid = false;
+  dst->tagsOfStep = dst->tagsOfStep && src->tagsOfStep;
   return LBM_OK;
 }
 

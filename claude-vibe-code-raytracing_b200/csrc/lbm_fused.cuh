@@ -407,13 +407,23 @@ __device__ __forceinline__ Real edot(Real X, Real Y, Real Z) {
   return r;
 }
 
+// gradient and laplacian of phi at a cell from its stencil values
+template <class PopT, class Real>
+__device__ __forceinline__ void phi_stencil(const CellLoad<PopT> &L, Real &gx, Real &gy, Real &gz, Real &lap) {
+  const Real half = (Real)0.5;
+  gx = rmul(half, rsub(L.pxp, L.pxm));
+  gy = rmul(half, rsub(L.pyp, L.pym));
+  gz = rmul(half, rsub(L.pzp, L.pzm));
+  lap = rfma((Real)-6, L.p, radd(radd(radd(radd(radd(L.pxp, L.pxm), L.pyp), L.pym), L.pzp), L.pzm));
+}
+
 // The collision of one cell into registers (o).  MODE 0: every direction (a
 // tile cell; opposite pairs evaluated together); MODE 1: the directions of the
 // compile-time halo side (SX, SY); MODE 2: every direction, one at a time (a
-// halo cell whose side is known at run time).  Returns gradient, laplacian
-// and   Every operation rounds explicitly (rmul / radd / rsub
-// / rfma), so a tile cell and a halo cell of another tile get the same bits
-// whatever the compiler would contract in either context.
+// halo cell whose side is known at run time).  Returns gradient and laplacian of
+// phi.  Every operation rounds explicitly (rmul / radd / rsub / rfma), so a tile
+// cell and a halo cell of another tile get the same bits whatever the compiler
+// would contract in either context.
 template <class PopT, int MODE, int SX, int SY>
 __device__ __forceinline__ void collide_cell(const CollK<typename Prec<PopT>::Real> &K, const CellLoad<PopT> &L,
                                              CellOut<PopT> &o, typename Prec<PopT>::Real &ogx,
@@ -426,11 +436,9 @@ __device__ __forceinline__ void collide_cell(const CollK<typename Prec<PopT>::Re
   const Real om = K.om, omP = K.omP, A = K.A, beta4 = K.beta4, kappa = K.kappa, rhoG = K.rhoG;
   const Real dRho = K.dRho, grav = K.grav, sharpC4 = K.sharpC4;
   const Real p = L.p, ux = L.ux, uy = L.uy, uz = L.uz;
-  const Real half = (Real)0.5, one = (Real)1, two = (Real)2;
-  const Real gxv = rmul(half, rsub(L.pxp, L.pxm));
-  const Real gyv = rmul(half, rsub(L.pyp, L.pym));
-  const Real gzv = rmul(half, rsub(L.pzp, L.pzm));
-  const Real lap = rfma((Real)-6, p, radd(radd(radd(radd(radd(L.pxp, L.pxm), L.pyp), L.pym), L.pzp), L.pzm));
+  const Real one = (Real)1, two = (Real)2;
+  Real gxv, gyv, gzv, lap;
+  phi_stencil(L, gxv, gyv, gzv, lap);
   const Real rhoPh = rfma(p, dRho, rhoG);
   const Real mu = rfma(-kappa, lap, rmul(rmul(rmul(beta4, p), rsub(p, one)), rfma(two, p, -one)));
   const Real Fx = rmul(mu, gxv), Fy = rfma(mu, gyv, rmul(rhoPh, grav)), Fz = rmul(mu, gzv);

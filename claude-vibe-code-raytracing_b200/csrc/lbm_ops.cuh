@@ -367,6 +367,7 @@ class Ops final : public OpsBase {
     a.ns = c.ns;
     a.redChunks = std::max(1, c.redChunks);
     a.listCap = (int)h->listCap;
+    a.anyTag = c.anyTag ? 1 : 0;
     a.ticket = h->redTickets;
     a.partials = h->partials;
     a.impulse = h->dOut;
@@ -382,6 +383,11 @@ class Ops final : public OpsBase {
   void shell(lbm_sim *h, const StepCtx &c) override {
     k_shell<PopT><<<dim3(std::max(1, c.redChunks), std::max(1, c.ns)), SHELL_THREADS, 0, h->stream>>>(
         make_shell(h, c, h->cur));
+    h->launches++;
+  }
+  void finish_unowned(lbm_sim *h) override {
+    k_finish_unowned<PopT><<<std::min(nblocks(h->n, 256), 148u * 8u), 256, 0, h->stream>>>(make_args(h, h->cur, 1),
+                                                                                         h->plan());
     h->launches++;
   }
   template <int TY, int STG, bool WIDE>

@@ -29,6 +29,7 @@ struct ShellArgs {
   const Plan *plan;   // this step's
   double rhoL;
   int ns, redChunks, listCap;  // chunks per sphere: redChunks blocks each
+  int anyTag;                  // the tags may not be the plan's: links anywhere in the spheres' boxes
   unsigned *ticket;
   double *partials, *impulse;  // per chunk; fluid [MAX][6], then dead-cell [MAX][6]
   const int *dead, *totals;
@@ -63,12 +64,69 @@ __device__ __forceinline__ int link_dir(int k) {
   return (ex + 1) | (ey + 1) << 2 | (ez + 1) << 4 | ((ex != 0) + (ey != 0) + (ez != 0)) << 6 | opp_of(k) << 8;
 }
 
+// the phi stencil of cell i (interior) from the half that the step read
+template <class PopT>
+__device__ __forceinline__ void load_stencil(const Scene<PopT, typename Prec<PopT>::Real> &s, int cur, long long i,
+                                             CellLoad<PopT> &L) {
+  const long long nx = s.nx, nxny = nx * s.ny;
+  const auto *phi = s.phi[cur] + i;
+  L.p = phi[0];
+  L.pxp = phi[1];
+  L.pxm = phi[-1];
+  L.pyp = phi[nx];
+  L.pym = phi[-nx];
+  L.pzp = phi[nxny];
+  L.pzm = phi[-nxny];
+}
+
+// The tiles leave the raw sums of every FLUID cell with a SOLID source; the
+// blocks below finish those with a source that a sphere of the plan contains.
+// Where the tags are not the plan's (written since the step's retag, or left by
+// a plan that ran out of room) there may be others: their SOLID sources are
+// walls at rest, so their populations are right and only the macros remain.
+template <class PopT>
+__device__ __forceinline__ void finish_unowned(const FusedArgs<PopT> &f, const SolidSet &ss, int x, int y, int z) {
+  using Real = typename Prec<PopT>::Real;
+  const auto &s = f.s;
+  const int cur = f.cur, nxt = 1 - cur;
+  const long long i = ((long long)z * s.ny + y) * s.nx + x;
+  if (s.tag[i] != TAG_FLUID) return;
+  bool raw = false;
+#pragma unroll 1
+  for (int k = 1; k < Q27; k++) {
+    const int sx = x - dcomp(k, 0), sy = y - dcomp(k, 1), sz = z - dcomp(k, 2);
+    if (s.tag[((long long)sz * s.ny + sy) * s.nx + sx] != TAG_SOLID) continue;
+    raw = true;
+    if (owner_of<LBM_MAX_SPHERES>(ss.sph, ss.nsph, sx, sy, sz) >= 0) return;
+  }
+  if (!raw) return;
+  CellLoad<PopT> L;
+  load_stencil(s, cur, i, L);
+  Real gx, gy, gz, lap, rho, ux, uy, uz;
+  phi_stencil(L, gx, gy, gz, lap);
+  finish_macros(coll_consts(f), s.phi[nxt][i], gx, gy, gz, lap, s.rho[nxt][i], s.ux_at(nxt, i), s.uy_at(nxt, i),
+                s.uz[nxt][i], rho, ux, uy, uz);
+  s.rho[nxt][i] = rho;
+  s.set_ux(nxt, i, ux);
+  s.set_uy(nxt, i, uy);
+  s.uz[nxt][i] = uz;
+}
+// the whole grid, after a step whose tags were written since its retag
+template <class PopT>
+__global__ void k_finish_unowned(const __grid_constant__ FusedArgs<PopT> f, const Plan *__restrict__ plan) {
+  const int nx = f.s.nx, ny = f.s.ny, nz = f.s.nz;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < f.s.n; i += (long long)gridDim.x * blockDim.x) {
+    const int t = (int)(i / nx), x = (int)(i - (long long)t * nx), z = t / ny, y = t - z * ny;
+    if (x >= 1 && x <= nx - 2 && y >= 1 && y <= ny - 2 && z >= 1 && z <= nz - 2) finish_unowned(f, plan->ss, x, y, z);
+  }
+}
+
 constexpr int SHELL_THREADS = 256;
 static_assert(SHELL_THREADS == RED_THREADS && SHELL_THREADS == DEAD_THREADS && SHELL_THREADS >= Q27, "");
 
 // Block (chunk cx of sphere b): 1,024 cells of the sphere's box in scan order.
-//   1. the cells with links to a SOLID cell are listed: only cells within
-//      sqrt(3) outside the sphere can have any;
+//   1. the cells with links to a SOLID cell are listed: where the tags are the
+//      plan's, only cells within sqrt(3) outside the sphere can have any;
 //   2. each listed cell is collided, one thread per cell; its momentum exchange
 //      with this sphere is summed in direction order into its slot, and the
 //      block of the first sphere that it has a link to adds the links'
@@ -108,7 +166,7 @@ __device__ __forceinline__ void shell_body(const ShellArgs<PopT> &a, int cx, int
     const int cells = (int)((long long)t.dim[0] * t.dim[1] * t.dim[2]), c0 = cx * RED_CHUNK;
     const int dxb = t.dim[0], dyb = t.dim[1], lo0 = t.lo[0], lo1 = t.lo[1], lo2 = t.lo[2];
     const double rIn = sp.r > 1.0 ? sp.r - 1.0 : 0.0, rOut = sp.r + 2.0;
-    const double in2 = rIn * rIn, out2 = rOut * rOut;
+    const double in2 = a.anyTag ? 0 : rIn * rIn, out2 = a.anyTag ? INFINITY : rOut * rOut;
     if (tid == 0) sCount = 0;
     if (tid < Q27) sDir[tid] = link_dir(tid);
     __syncthreads();
@@ -162,14 +220,7 @@ __device__ __forceinline__ void shell_body(const ShellArgs<PopT> &a, int cx, int
           });
         }
       });
-      const Real *phi = s.phi[cur] + i;
-      L.p = phi[0];
-      L.pxp = phi[1];
-      L.pxm = phi[-1];
-      L.pyp = phi[nx];
-      L.pym = phi[-nx];
-      L.pzp = phi[nxny];
-      L.pzm = phi[-nxny];
+      load_stencil(s, cur, i, L);
       L.sumF = s.rho[cur][i];
       L.ux = s.ux_at(cur, i);
       L.uy = s.uy_at(cur, i);

@@ -81,6 +81,7 @@ inline bool needs_wide(long long cells) { return pop_elems(cells, 27) >= (1LL <<
 struct StepCtx {
   int ns = 0, redChunks = 0;
   bool tail = false;
+  bool anyTag = false;  // the tags may not be the plan's
   long long slotCells = 0, maxU = 0;
 };
 
@@ -111,6 +112,7 @@ class OpsBase {
   virtual void absorb_dead(lbm_sim *h, double *d_out) = 0;
   virtual void fused_step(lbm_sim *h, const FusedCfg &cfg) = 0;
   virtual void shell(lbm_sim *h, const StepCtx &c) = 0;  // after fused_step, before cur flips
+  virtual void finish_unowned(lbm_sim *h) = 0;           // after shell, where the tags may not be the plan's
   virtual void pack(lbm_sim *h, uint8_t *d_out) = 0;
   virtual void pack_end_planes(lbm_sim *h, uint8_t *d_out) = 0;
   virtual void watch_finite(lbm_sim *h, unsigned long long *d_first) = 0;
@@ -253,6 +255,9 @@ struct lbm_sim {
   bool sequentialFill = false;
   int stepBegunNs = -1;
   bool planOfStep = false;  // the device plan is the begun step's
+  // no tag has been written since the last step's retag (planes copied from
+  // another slab of the scene are that slab's)
+  bool tagsOfStep = false;
   // a SOLID cell may differ between the halves (a field write, a phase-by-phase
   // call): carried over the whole grid before the next fused step
   bool carrySolid = false;
