@@ -605,6 +605,7 @@ int coupled_prepare(lbm_sim *h, const lbm_sphere *sp, int ns, bool frames, Coupl
   memset(&h->hPlan, 0, sizeof(Plan));
   h->hPlan.boxLast = h->boxLast;
   h->hPlan.boxLastLast = h->boxLastLast;
+  h->hPlan.stale = Box{{1, 1, 1}, {0, 0, 0}};
   h->hPlan.fullRetag = h->fullRetagSteps;
   h->hPlan.ss.nsph = ns;
   if ((rc = upload_plan(h))) return rc;
@@ -647,7 +648,10 @@ int coupled_finish(lbm_sim *h, lbm_sphere *sp, int ns, int nsteps) {
   h->fullRetagSteps = h->hPlan.fullRetag;
   h->lastRetagBox = h->hPlan.U;
   h->listsValid = true;
-  if (h->hPlan.overflow) return fail(h, LBM_ERR_CAPACITY, "sphere moved beyond the planned retag box");
+  if (h->hPlan.overflow) {
+    h->fullRetagSteps = 2;  // SOLID cells may be left anywhere
+    return fail(h, LBM_ERR_CAPACITY, "sphere moved beyond the planned retag box");
+  }
   return LBM_OK;
 }
 

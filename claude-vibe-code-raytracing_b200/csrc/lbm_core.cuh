@@ -388,6 +388,7 @@ struct Plan {
   Box boxLast, boxLastLast;  // sphere boxes of the two previous retags
   int fullRetag;             // retag the whole grid for this many more steps
   int overflow;              // the plan exceeded the launch capacity
+  Box stale;                 // device-resident loop: SOLID cells that steps with no room to retag left behind
 };
 
 

@@ -823,6 +823,7 @@ __device__ __forceinline__ void plan_body(Plan *P, const Plan *prev, const lbm_s
   const Box boxLast = prev->boxLast, boxLastLast = prev->boxLastLast;
   const int fullRetag = prev->fullRetag;
   int overflow = prev->overflow;
+  Box stale = prev->stale;
   ss.nsph = nsph;
   ss.zlo = ss.zend = 0;
   Box now{{1, 1, 1}, {0, 0, 0}};
@@ -869,10 +870,12 @@ __device__ __forceinline__ void plan_body(Plan *P, const Plan *prev, const lbm_s
   long long uc = box_cells(U);
   if (uc > maxUCells) {
     overflow = 1;
+    stale = box_union(stale, boxLast);
     uc = 0;
     U = Box{{1, 1, 1}, {0, 0, 0}};
   }
   P->overflow = overflow;
+  P->stale = stale;
   P->U = U;
   P->ucells = uc;
   P->nchunks = (int)((uc + COMPACT_CHUNK - 1) / COMPACT_CHUNK);

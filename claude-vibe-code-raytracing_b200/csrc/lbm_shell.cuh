@@ -166,7 +166,8 @@ __device__ __forceinline__ void shell_body(const ShellArgs<PopT> &a, int cx, int
     const int cells = (int)((long long)t.dim[0] * t.dim[1] * t.dim[2]), c0 = cx * RED_CHUNK;
     const int dxb = t.dim[0], dyb = t.dim[1], lo0 = t.lo[0], lo1 = t.lo[1], lo2 = t.lo[2];
     const double rIn = sp.r > 1.0 ? sp.r - 1.0 : 0.0, rOut = sp.r + 2.0;
-    const double in2 = a.anyTag ? 0 : rIn * rIn, out2 = a.anyTag ? INFINITY : rOut * rOut;
+    const bool anyTag = a.anyTag || a.plan->overflow;
+    const double in2 = anyTag ? 0 : rIn * rIn, out2 = anyTag ? INFINITY : rOut * rOut;
     if (tid == 0) sCount = 0;
     if (tid < Q27) sDir[tid] = link_dir(tid);
     __syncthreads();
@@ -338,6 +339,16 @@ __device__ __forceinline__ void shell_body(const ShellArgs<PopT> &a, int cx, int
     for (int sb = 0; sb < ns; sb++)
       absorb_dead_body(SceneFields<PopT>{s, cur}, nx, ny, a.dead, a.totals, a.listCap, a.rhoL, a.f.rhoG, &ss,
                        a.impulse + LBM_MAX_SPHERES * 6, sb, sh);
+    if (a.plan->overflow) {
+      // the run is reported as failed; its fields stay those of a step next to
+      // walls at rest where the old SOLID cells are
+      const Box w = box_grow(a.plan->stale, 1, nx, ny, nz);
+      const int dx = w.hi[0] - w.lo[0] + 1, dy = w.hi[1] - w.lo[1] + 1, n = (int)box_cells(w);
+      for (int c = tid; c < n; c += SHELL_THREADS) {
+        const int q = c / dx, x = w.lo[0] + c - q * dx, y = w.lo[1] + q % dy, z = w.lo[2] + q / dy;
+        if (x >= 1 && x <= nx - 2 && y >= 1 && y <= ny - 2 && z >= 1 && z <= nz - 2) finish_unowned(a.f, ss, x, y, z);
+      }
+    }
     __syncthreads();
     if (a.sph && tid < ns)
       sphere_step_body(a.sph, tid, a.f.gravity, a.impulse, a.impulse + LBM_MAX_SPHERES * 6, nx, ny, nz);
