@@ -124,6 +124,21 @@ __global__ void k_finish_unowned(const __grid_constant__ FusedArgs<PopT> f, cons
 constexpr int SHELL_THREADS = 256;
 static_assert(SHELL_THREADS == RED_THREADS && SHELL_THREADS == DEAD_THREADS && SHELL_THREADS >= Q27, "");
 
+// A plan without room for the retag (the run is reported as failed): the fields
+// stay those of a step next to walls at rest where the old SOLID cells are.
+// (Not inlined: in the shell's body it cost 0.5 us of 41 a step at 40x28x40.)
+template <class PopT>
+__device__ __noinline__ void finish_stale(const ShellArgs<PopT> &a) {
+  const auto &s = a.f.s;
+  const Box w = box_grow(a.plan->stale, 1, s.nx, s.ny, s.nz);
+  const int dx = w.hi[0] - w.lo[0] + 1, dy = w.hi[1] - w.lo[1] + 1, n = (int)box_cells(w);
+  for (int c = threadIdx.x; c < n; c += SHELL_THREADS) {
+    const int q = c / dx, x = w.lo[0] + c - q * dx, y = w.lo[1] + q % dy, z = w.lo[2] + q / dy;
+    if (x >= 1 && x <= s.nx - 2 && y >= 1 && y <= s.ny - 2 && z >= 1 && z <= s.nz - 2)
+      finish_unowned(a.f, a.plan->ss, x, y, z);
+  }
+}
+
 // Block (chunk cx of sphere b): 1,024 cells of the sphere's box in scan order.
 //   1. the cells with links to a SOLID cell are listed: where the tags are the
 //      plan's, only cells within sqrt(3) outside the sphere can have any;
@@ -153,7 +168,7 @@ __device__ __forceinline__ void shell_body(const ShellArgs<PopT> &a, int cx, int
   const auto &s = a.f.s;
   const int tid = threadIdx.x;
   const int nx = s.nx, ny = s.ny, nz = s.nz, nxny = nx * ny, cur = a.f.cur, nxt = 1 - cur;
-  const int ns = ss.nsph;
+  const int ns = ss.nsph, over = a.plan->overflow;
   auto chunks_of = [&](int j) {
     const ImpulseTarget &t = ss.imp[j];
     const long long cells = (long long)t.dim[0] * t.dim[1] * t.dim[2];
@@ -166,7 +181,7 @@ __device__ __forceinline__ void shell_body(const ShellArgs<PopT> &a, int cx, int
     const int cells = (int)((long long)t.dim[0] * t.dim[1] * t.dim[2]), c0 = cx * RED_CHUNK;
     const int dxb = t.dim[0], dyb = t.dim[1], lo0 = t.lo[0], lo1 = t.lo[1], lo2 = t.lo[2];
     const double rIn = sp.r > 1.0 ? sp.r - 1.0 : 0.0, rOut = sp.r + 2.0;
-    const bool anyTag = a.anyTag || a.plan->overflow;
+    const bool anyTag = a.anyTag || over;
     const double in2 = anyTag ? 0 : rIn * rIn, out2 = anyTag ? INFINITY : rOut * rOut;
     if (tid == 0) sCount = 0;
     if (tid < Q27) sDir[tid] = link_dir(tid);
@@ -339,16 +354,7 @@ __device__ __forceinline__ void shell_body(const ShellArgs<PopT> &a, int cx, int
     for (int sb = 0; sb < ns; sb++)
       absorb_dead_body(SceneFields<PopT>{s, cur}, nx, ny, a.dead, a.totals, a.listCap, a.rhoL, a.f.rhoG, &ss,
                        a.impulse + LBM_MAX_SPHERES * 6, sb, sh);
-    if (a.plan->overflow) {
-      // the run is reported as failed; its fields stay those of a step next to
-      // walls at rest where the old SOLID cells are
-      const Box w = box_grow(a.plan->stale, 1, nx, ny, nz);
-      const int dx = w.hi[0] - w.lo[0] + 1, dy = w.hi[1] - w.lo[1] + 1, n = (int)box_cells(w);
-      for (int c = tid; c < n; c += SHELL_THREADS) {
-        const int q = c / dx, x = w.lo[0] + c - q * dx, y = w.lo[1] + q % dy, z = w.lo[2] + q / dy;
-        if (x >= 1 && x <= nx - 2 && y >= 1 && y <= ny - 2 && z >= 1 && z <= nz - 2) finish_unowned(a.f, ss, x, y, z);
-      }
-    }
+    if (over) finish_stale(a);
     __syncthreads();
     if (a.sph && tid < ns)
       sphere_step_body(a.sph, tid, a.f.gravity, a.impulse, a.impulse + LBM_MAX_SPHERES * 6, nx, ny, nz);
