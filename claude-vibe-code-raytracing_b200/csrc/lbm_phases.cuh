@@ -60,6 +60,14 @@ __device__ __forceinline__ void store_groups(PopT *p, const PopT (&v)[PopGroups<
   });
 }
 
+// e.X with every term, as the reference has it: 0 * X is NaN where X is not
+// finite, so a blow-up in one component reaches every direction (edot skips
+// those terms)
+template <int ex, int ey, int ez, class Real>
+__device__ __forceinline__ Real edot_all(Real X, Real Y, Real Z) {
+  return rfma((Real)ez, Z, rfma((Real)ey, Y, rmul((Real)ex, X)));
+}
+
 // computePhiGradients (src/sim.js:176-199)
 template <class PopT>
 __global__ void __launch_bounds__(PHASE_THREADS) k_gradients(Scene<PopT, typename Prec<PopT>::Real> s, int cur) {
@@ -106,9 +114,9 @@ __global__ void __launch_bounds__(PHASE_THREADS)
     constexpr int q = decltype(KK)::value;
     using D = D7<q>;
     const Real wk = (Real)D::w;
-    const Real eu = edot<D::ex, D::ey, D::ez>(uxi, uyi, uzi);
+    const Real eu = edot_all<D::ex, D::ey, D::ez>(uxi, uyi, uzi);
     const Real heq = wk * p * ((Real)1 + (Real)4 * eu);
-    const Real Fk = wk * edot<D::ex, D::ey, D::ez>(Sx, Sy, Sz);
+    const Real Fk = wk * edot_all<D::ex, D::ey, D::ez>(Sx, Sy, Sz);
     const Real hk = (Real)h[q];
     h[q] = (PopT)(hk - invTau * (hk - heq) + Fk);
   });
@@ -177,10 +185,10 @@ __global__ void __launch_bounds__(PHASE_THREADS)
     constexpr int q = decltype(KK)::value;
     using D = D27<q>;
     const Real wk = (Real)D::w;
-    const Real eu = edot<D::ex, D::ey, D::ez>(uxe, uye, uze);
+    const Real eu = edot_all<D::ex, D::ey, D::ez>(uxe, uye, uze);
     const Real Qi = negU2half + eu * ((Real)3 + (Real)4.5 * eu);
     const Real feq = wk * (sumF + rhoPhase * Qi);
-    const Real ekF = edot<D::ex, D::ey, D::ez>(fx, fy, fz);
+    const Real ekF = edot_all<D::ex, D::ey, D::ez>(fx, fy, fz);
     const Real Sk = A * wk * (ekF * ((Real)1 + (Real)3 * eu) - uF);
     const Real fk = (Real)f[q];
     f[q] = (PopT)(fk - invTau * (fk - feq) + Sk);
@@ -235,9 +243,9 @@ __global__ void __launch_bounds__(PHASE_THREADS)
       last[q & 3] = v[q];
       if constexpr ((q & 3) == 3) st4_global(f + 32 * (q >> 2), last);
       pSumF += fk;
-      if constexpr (D::ex != 0) mx = D::ex > 0 ? mx + fk : mx - fk;
-      if constexpr (D::ey != 0) my = D::ey > 0 ? my + fk : my - fk;
-      if constexpr (D::ez != 0) mz = D::ez > 0 ? mz + fk : mz - fk;
+      mx = rfma((Real)D::ex, fk, mx);
+      my = rfma((Real)D::ey, fk, my);
+      mz = rfma((Real)D::ez, fk, mz);
     });
   } else {
     const SolidSet &ss = *ssp;
