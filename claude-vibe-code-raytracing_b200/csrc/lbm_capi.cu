@@ -2109,8 +2109,10 @@ int lbm_batch_run(lbm_batch *b, lbm_sphere *const *spheres, const int *nspheres,
   std::vector<unsigned char> small(shellOff + 2 * (size_t)n * hb);
   long long maxChunks = 1;
   int redX = 1, nsMax = 0;
+  bool inOrder = false;
   for (int s = 0; s < n; s++) {
     lbm_sim *h = b->sims[s];
+    inOrder = inOrder || h->sequentialFill;
     for (int p = 0; p < 2; p++) {
       ops->small_args(h, h->cur ^ p, &small[((size_t)p * n + s) * sb]);
       ops->shell_args(h, ctx[s], h->cur ^ p, &small[shellOff + ((size_t)p * n + s) * hb]);
@@ -2151,7 +2153,7 @@ int lbm_batch_run(lbm_batch *b, lbm_sphere *const *spheres, const int *nspheres,
   // scenes, around the shared fused launch, all on the batch's stream
   auto emit_step = [&](int parity) -> int {
     const void *A = (const unsigned char *)b->dSmall + (size_t)parity * n * sb;
-    ops->batch_sets(A, n, setCtas, b->origin);
+    ops->batch_sets(A, n, setCtas, inOrder, b->origin);
     BCK(cudaGetLastError());
     ops->fused_batch((const unsigned char *)b->dArgs + (size_t)parity * n * ab, b->dTileStart, b->dTileGrid,
                      n, launch_shape(b, b->rows), ctas, b->origin);
@@ -2193,7 +2195,7 @@ int lbm_batch_run(lbm_batch *b, lbm_sphere *const *spheres, const int *nspheres,
   if (graph) {
     std::vector<long long> key = {b->rows, b->zchunk, (long long)(uintptr_t)b->dArgs,
                                   (long long)(uintptr_t)b->dTileStart, ctas, (long long)(uintptr_t)b->dSmall,
-                                  setCtas, redX, nsMax};
+                                  setCtas, redX, nsMax, inOrder};
     for (int s = 0; s < n; s++) {
       lbm_sim *h = b->sims[s];
       const long long v[] = {(long long)(uintptr_t)h,           h->cur,      ctx[s].ns,

@@ -196,7 +196,7 @@ __device__ __forceinline__ void box_cell(const Box &bx, long long l, int &x, int
 // between the cells of a group is kept by rounds: a cell is filled in the first
 // round in which its fresh neighbours before it have been filled.  A z slab
 // fills its own planes only (its copied planes receive the neighbouring slab's
-// filled values).  sequential != 0: one cell at a time.
+// filled values).
 // Latency-bound: with a thread per cell that went from neighbour to neighbour,
 // one fresh cell took 31,000 cycles and twenty 75,000 to 118,000 (256^3, one
 // sphere of radius 24); now 6,600, and 10,000 to 15,000.
@@ -205,7 +205,7 @@ constexpr int FILL_GROUP = 32;
 template <class PopT, int THREADS>
 __device__ __forceinline__ void fresh_fill_body(const Scene<PopT, typename Prec<PopT>::Real> &s, int cur,
                                                 const int *fresh, int nf, double rhoL, double rhoG, int zlo,
-                                                int zend, int sequential) {
+                                                int zend) {
   using Real = typename Prec<PopT>::Real;
   constexpr int WARPS = THREADS / 32, OWN = 13;  // (neighbour 13 is the cell itself)
   static_assert(FILL_GROUP == 32 && FILL_GROUP % WARPS == 0 && THREADS >= 5 * FILL_GROUP, "");
@@ -221,9 +221,8 @@ __device__ __forceinline__ void fresh_fill_body(const Scene<PopT, typename Prec<
   const int k = min(lane, Q27 - 1);  // the lane's direction
   const double ex = dcomp(k, 0), ey = dcomp(k, 1), ez = dcomp(k, 2);
   const float w = w27_of(k), w7 = w7_of(min(k, Q7 - 1));
-  const int group = sequential ? 1 : FILL_GROUP;
-  for (int g0 = 0; g0 < nf; g0 += group) {
-    const int m = min(group, nf - g0);
+  for (int g0 = 0; g0 < nf; g0 += FILL_GROUP) {
+    const int m = min(FILL_GROUP, nf - g0);
     if (threadIdx.x < FILL_GROUP) {
       int i = -1;
       if (lane < m) {
@@ -308,6 +307,51 @@ __device__ __forceinline__ void fresh_fill_body(const Scene<PopT, typename Prec<
       }
     }
     __syncthreads();
+  }
+}
+
+// The same as the reference's loop, in place by one thread in list order: the
+// test hook's fill (lbm_test_sequential_fill), which shares nothing with the
+// one above.
+template <class PopT>
+__device__ __forceinline__ void fresh_fill_in_order(const Scene<PopT, typename Prec<PopT>::Real> &s, int cur,
+                                                    const int *fresh, int nf, double rhoL, double rhoG, int zlo,
+                                                    int zend) {
+  using Real = typename Prec<PopT>::Real;
+  const long long nxny = (long long)s.nx * s.ny;
+  for (int q = 0; q < nf; q++) {
+    const long long i = fresh[q], z = i / nxny;
+    if (zend > 0 && (z < zlo || z >= zend)) continue;
+    double ps = 0, rs = 0, xs = 0, ys = 0, zs = 0;
+    int cnt = 0;
+    for (int dz = -1; dz <= 1; dz++)
+      for (int dy = -1; dy <= 1; dy++)
+        for (int dx = -1; dx <= 1; dx++) {
+          const long long j = i + dz * nxny + (long long)dy * s.nx + dx;
+          if (j == i || s.tag[j] != TAG_FLUID) continue;
+          ps += (double)s.phi[cur][j];
+          rs += (double)s.rho[cur][j];
+          xs += (double)s.ux_at(cur, j);
+          ys += (double)s.uy_at(cur, j);
+          zs += (double)s.uz[cur][j];
+          cnt++;
+        }
+    const double p = cnt ? ps / cnt : (double)s.phi[cur][i], r = cnt ? rs / cnt : 1.0;
+    const double vx = cnt ? xs / cnt : 0.0, vy = cnt ? ys / cnt : 0.0, vz = cnt ? zs / cnt : 0.0;
+    s.phi[0][i] = s.phi[1][i] = (Real)p;
+    s.rho[cur][i] = (Real)r;
+    s.set_ux(cur, i, (Real)vx);
+    s.set_uy(cur, i, (Real)vy);
+    s.uz[cur][i] = (Real)vz;
+    const double rhoPhase = rhoG + p * (rhoL - rhoG), u2 = vx * vx + vy * vy + vz * vz;
+    for (int k = 0; k < Q27; k++) {
+      const double eu = dcomp(k, 0) * vx + dcomp(k, 1) * vy + dcomp(k, 2) * vz;
+      const double fk = (double)w27_of(k) * (r + rhoPhase * (eu * (3.0 + 4.5 * eu) - 1.5 * u2));
+      s.F[cur][pidx<27>(k, i)] = Codec<PopT>::enc((Real)fk, (Real)w27_of(k));
+      if (k < Q7)
+        s.H[cur][pidx<7>(k, i)] =
+            Codec<PopT>::enc((Real)((double)w7_of(k) * p * (1 + 4.0 * eu)), (Real)w7_of(k) * (Real)p);
+    }
   }
 }
 
@@ -526,8 +570,8 @@ __device__ __forceinline__ void sets_body(const SmallArgs<PopT> &a, unsigned bid
     a.totals[1] = all.y;
   }
   if constexpr (FILL) {
-    if (all.x == 0) return;
-    fresh_fill_body<PopT, SETS_THREADS>(s, a.cur, a.fresh, min(all.x, a.listCap), a.rhoL, a.rhoG, a.zlo, a.zend, a.seqFill);
+    if (all.x == 0 || a.seqFill) return;
+    fresh_fill_body<PopT, SETS_THREADS>(s, a.cur, a.fresh, min(all.x, a.listCap), a.rhoL, a.rhoG, a.zlo, a.zend);
   }
 }
 template <class PopT, bool RETAG, bool FILL>
@@ -540,11 +584,21 @@ __global__ void __launch_bounds__(SETS_THREADS) kb_sets(const SmallArgs<PopT> *_
   sets_body<PopT, true, true>(A[blockIdx.y], blockIdx.x, gridDim.x);
 }
 
-// absorbDeadCells (src/solid.js:87-101): impulse rho(phi)*u of every cell on
-// the scan-ordered dead list, in FP64, to the sphere owning the cell.  One CTA
-// per sphere; thread t sums the contiguous t-th share of the list in scan
-// order, then a fixed shared-memory tree adds the shares -- deterministic,
-// and independent of how many dead cells there are per step.
+// with the test hook on, after k_sets / kb_sets; scene b in block b
+template <class PopT>
+__device__ __forceinline__ void fill_in_order_body(const SmallArgs<PopT> &a) {
+  if (a.seqFill && threadIdx.x == 0)
+    fresh_fill_in_order<PopT>(a.s, a.cur, a.fresh, min(a.totals[0], a.listCap), a.rhoL, a.rhoG, a.zlo, a.zend);
+}
+template <class PopT>
+__global__ void k_fill_in_order(const __grid_constant__ SmallArgs<PopT> a) {
+  fill_in_order_body<PopT>(a);
+}
+template <class PopT>
+__global__ void kb_fill_in_order(const SmallArgs<PopT> *__restrict__ A) {
+  fill_in_order_body<PopT>(A[blockIdx.x]);
+}
+
 // ---------------------------------------------------------------- generic solids
 // retagCells(solid) for any duck-typed solid (src/sim.js:214-244): the host
 // has evaluated solid.contains / solid.surfaceVelocity per cell into mask
@@ -670,6 +724,11 @@ __global__ void __launch_bounds__(LINK_CHUNK) k_link_emit(Scene<PopT, typename P
   }
 }
 
+// absorbDeadCells (src/solid.js:87-101): impulse rho(phi)*u of every cell on
+// the scan-ordered dead list, in FP64, to the sphere owning the cell.  One CTA
+// per sphere; thread t sums the contiguous t-th share of the list in scan
+// order, then a fixed shared-memory tree adds the shares -- deterministic,
+// and independent of how many dead cells there are per step.
 constexpr int DEAD_THREADS = 256;
 
 // (static: Real = float is instantiated by several translation units)

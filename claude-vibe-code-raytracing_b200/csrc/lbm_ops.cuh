@@ -239,6 +239,10 @@ class Ops final : public OpsBase {
     else if (fill) k_sets<PopT, false, true><<<ctas, SETS_THREADS, 0, h->stream>>>(a);
     else k_sets<PopT, false, false><<<ctas, SETS_THREADS, 0, h->stream>>>(a);
     h->launches++;
+    if (fill && h->sequentialFill) {
+      k_fill_in_order<PopT><<<1, 32, 0, h->stream>>>(a);
+      h->launches++;
+    }
   }
   void absorb_dead(lbm_sim *h, double *d_out) override {
     const int ns = h->hPlan.ss.nsph > 0 ? h->hPlan.ss.nsph : 1;
@@ -473,8 +477,9 @@ class Ops final : public OpsBase {
   void batch_plan(const void *d_shell, int n, cudaStream_t st) override {
     kb_plan<PopT><<<n, 32, 0, st>>>((const ShellArgs<PopT> *)d_shell);
   }
-  void batch_sets(const void *d_small, int n, unsigned ctas, cudaStream_t st) override {
+  void batch_sets(const void *d_small, int n, unsigned ctas, bool inOrder, cudaStream_t st) override {
     kb_sets<PopT><<<dim3(ctas, n), SETS_THREADS, 0, st>>>((const SmallArgs<PopT> *)d_small);
+    if (inOrder) kb_fill_in_order<PopT><<<n, 32, 0, st>>>((const SmallArgs<PopT> *)d_small);
   }
   void batch_shell(const void *d_shell, int n, int redChunks, int spheres, cudaStream_t st) override {
     kb_shell<PopT><<<dim3(redChunks, std::max(1, spheres), n), SHELL_THREADS, 0, st>>>(

@@ -156,7 +156,8 @@ class OpsBase {
   virtual void small_args(lbm_sim *h, int cur, void *out) = 0;
   virtual void shell_args(lbm_sim *h, const StepCtx &c, int cur, void *out) = 0;
   virtual void batch_plan(const void *d_shell, int n, cudaStream_t st) = 0;
-  virtual void batch_sets(const void *d_small, int n, unsigned ctas, cudaStream_t st) = 0;
+  // (inOrder: a scene has the test hook's fill)
+  virtual void batch_sets(const void *d_small, int n, unsigned ctas, bool inOrder, cudaStream_t st) = 0;
   virtual void batch_shell(const void *d_shell, int n, int redChunks, int spheres, cudaStream_t st) = 0;
   // the tensor maps of the TMA-staged form (h->dMaps), where the storage
   // form and the grid allow them (nx a multiple of 16); none otherwise
