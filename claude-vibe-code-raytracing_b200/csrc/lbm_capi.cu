@@ -355,9 +355,17 @@ void set_box(lbm_sim *h, const Box &bx) {
   h->hPlan.nchunks = (int)((h->hPlan.ucells + COMPACT_CHUNK - 1) / COMPACT_CHUNK);
 }
 
-// fresh / dead lists over a box, scan order, and the fresh fill (fill)
+// fresh / dead lists over a box, scan order, and the fresh fill (fill).  Cells of
+// the domain's faces are neither, whatever tags were written (src/sim.js:259,
+// src/solid.js:89: both loops run over 1 .. n-2): a fill reads 26 neighbours.
 int compact_sets(lbm_sim *h, const Box &bx, bool fill) {
-  set_box(h, bx);
+  Box in = bx;
+  const Box inner = interior(h);
+  for (int a = 0; a < 3; a++) {
+    in.lo[a] = std::max(in.lo[a], inner.lo[a]);
+    in.hi[a] = std::min(in.hi[a], inner.hi[a]);
+  }
+  set_box(h, in);
   int rc = upload_plan(h);
   if (rc) return rc;
   return launch_sets(h, h->hPlan.nchunks, false, fill);
