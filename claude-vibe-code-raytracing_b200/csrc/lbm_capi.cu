@@ -591,7 +591,7 @@ int coupled_prepare(lbm_sim *h, const lbm_sphere *sp, int ns, bool frames, Coupl
   if (h->bfActive) return fail(h, LBM_ERR_STATE, "a pending body force needs lbm_step");
   if (!h->fusedOK) return fail(h, LBM_ERR_UNSUPPORTED, "grid too large for the fused kernel");
   double rmax = 0;
-  for (int b = 0; b < ns; b++) rmax = std::max(rmax, sp[b].r);
+  for (int b = 0; b < ns; b++) rmax = std::max(rmax, fabs(sp[b].r));
   long long side = 2 * (long long)ceil(rmax) + 7;
   c.ns = ns;
   c.slotCells = std::min(h->n, side * side * side);

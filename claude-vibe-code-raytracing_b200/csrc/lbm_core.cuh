@@ -307,6 +307,7 @@ __host__ __device__ inline Box sphere_box(double cx, double cy, double cz, doubl
   Box b;
   double c[3] = {cx, cy, cz};
   int n[3] = {nx, ny, nz};
+  r = fabs(r);  // contains compares squares
   for (int a = 0; a < 3; a++) {
     double lo = c[a] - r - 0.5, hi = c[a] + r - 0.5;
     // one cell of slack on each side against rounding at the boundary

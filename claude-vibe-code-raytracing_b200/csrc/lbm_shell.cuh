@@ -180,7 +180,7 @@ __device__ __forceinline__ void shell_body(const ShellArgs<PopT> &a, int cx, int
     const SphereDesc sp = ss.sph[b];
     const int cells = (int)((long long)t.dim[0] * t.dim[1] * t.dim[2]), c0 = cx * RED_CHUNK;
     const int dxb = t.dim[0], dyb = t.dim[1], lo0 = t.lo[0], lo1 = t.lo[1], lo2 = t.lo[2];
-    const double rIn = sp.r > 1.0 ? sp.r - 1.0 : 0.0, rOut = sp.r + 2.0;
+    const double rad = fabs(sp.r), rIn = rad > 1.0 ? rad - 1.0 : 0.0, rOut = rad + 2.0;
     const bool anyTag = a.anyTag || over;
     const double in2 = anyTag ? 0 : rIn * rIn, out2 = anyTag ? INFINITY : rOut * rOut;
     if (tid == 0) sCount = 0;
