@@ -47,7 +47,7 @@ from . import autotune, workloads
 from ._capi import STORAGE, lib
 from .batch import Batch
 
-# per-scene working buffers beyond lbm_footprint_bytes: compaction counts,
+# per-scene working buffers beyond lbm_footprint_bytes: compaction counts and words,
 # impulse slots, the frame staging buffer and the device plan (generous)
 _EXTRA_PER_CELL = 8
 _EXTRA_FIXED = 32 << 20

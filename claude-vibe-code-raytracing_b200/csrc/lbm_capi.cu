@@ -174,8 +174,9 @@ int upload_plan(lbm_sim *h) {
   return LBM_OK;
 }
 
-// The spheres' work arrays, in doubles: impulse slots and the partials of their
-// sums, grown on the handle's stream.
+// The spheres' work arrays, in doubles: impulse slots (grown by half, a box
+// changes from step to step) and the partials of their sums, on the handle's
+// stream.
 int ensure_work(lbm_sim *h, long long slots, long long partials) {
   const struct {
     double **p;
@@ -189,7 +190,7 @@ int ensure_work(lbm_sim *h, long long slots, long long partials) {
       *a.p = nullptr;
       *a.cap = 0;
     }
-    const long long cap = a.need + a.need / 2;
+    const long long cap = a.p == &h->impAcc ? a.need + a.need / 2 : a.need;
     DALLOC(*a.p, cap * sizeof(double));
     *a.cap = cap;
   }
@@ -269,6 +270,8 @@ int reduce_impulses(lbm_sim *h, double *d_out) {
   return LBM_OK;
 }
 
+// Per chunk of a retag box: counts and ballot words, grown by half, but no
+// further than the whole grid's chunks (0.25 bytes a cell).
 int ensure_counts(lbm_sim *h, long long nch) {
   if (nch <= h->countsCap) return LBM_OK;
   const size_t bits = SETS_WORDS * 2 * sizeof(uint32_t);
@@ -278,7 +281,7 @@ int ensure_counts(lbm_sim *h, long long nch) {
   h->counts = nullptr;
   h->setBits = nullptr;
   h->countsCap = 0;
-  const long long cap = nch + nch / 2;
+  const long long cap = std::max(nch, std::min(nch + nch / 2, (h->n + COMPACT_CHUNK - 1) / COMPACT_CHUNK));
   DALLOC(h->counts, cap * sizeof(int2));
   DALLOC(h->setBits, cap * bits);
   h->countsCap = cap;
