@@ -128,6 +128,7 @@ _SIGS = [
     ("lbm_fault_record", C.c_int, [C.c_void_p, C.POINTER(C.c_int64)]),
     ("lbm_test_withhold_stage_copy", C.c_int, [C.c_void_p, C.c_int]),
     ("lbm_test_sequential_fill", C.c_int, [C.c_void_p, C.c_int]),
+    ("lbm_test_ring_copies", C.c_int, [C.POINTER(C.c_int64)]),
     ("lbm_set_nan_watchdog", C.c_int, [C.c_void_p, C.c_int]),
     ("lbm_transfer_bytes", C.c_int, [C.c_void_p, C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)]),
     ("lbm_fused_timing", C.c_int, [C.c_void_p, C.c_int]),

@@ -1551,6 +1551,12 @@ int lbm_trim_device_memory(int device) {
   return cudaMemPoolTrimTo(pool, 0) == cudaSuccess ? LBM_OK : LBM_ERR_CUDA;
 }
 
+int lbm_test_ring_copies(int64_t *count) {
+  if (!count) return LBM_ERR_ARG;
+  *count = host_ring().copies;
+  return LBM_OK;
+}
+
 int lbm_host_alloc(size_t bytes, void **out) {
   if (!out || bytes == 0) return LBM_ERR_ARG;
   *out = nullptr;

@@ -64,6 +64,7 @@ inline void hostcopy_run(int n, F &f) {
 struct HostRing {
   std::mutex mu;
   std::atomic<int> handles{0};
+  std::atomic<long long> copies{0};  // that went through the ring (lbm_test_ring_copies)
   char *buf = nullptr;
   cudaEvent_t ev[HOSTCOPY_SLOTS] = {};
   int device = -1;  // the events'
@@ -176,6 +177,7 @@ inline cudaError_t copy_to_host(void *dst, const void *src, size_t bytes, int de
     if (e == cudaSuccess) e = e2;
     return e != cudaSuccess ? e : runtime();
   }
+  r.copies++;
   return cudaSuccess;
 }
 

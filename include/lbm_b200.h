@@ -318,6 +318,11 @@ int lbm_test_withhold_stage_copy(lbm_sim *sim, int on);
  * loop), instead of in parallel rounds; the results are the same bit for bit
  * either way. */
 int lbm_test_sequential_fill(lbm_sim *sim, int on);
+/* For the tests of large results (16 MB and more) into pageable memory: how
+ * many of them this process has copied by several threads out of the
+ * page-locked ring (the others, on machines with fewer than four cores or while
+ * another thread has the ring, went through the runtime's copy). */
+int lbm_test_ring_copies(int64_t *count);
 /* Host->device and device->host bytes this handle has copied since creation. */
 int lbm_transfer_bytes(const lbm_sim *sim, uint64_t *h2d, uint64_t *d2h);
 /* Time the fused step kernel with CUDA events on the handle's stream.
