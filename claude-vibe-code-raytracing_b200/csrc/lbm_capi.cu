@@ -248,8 +248,6 @@ int set_solids(lbm_sim *h, const lbm_sphere *sp, int ns, bool targets, bool clea
     off += cells;
     maxChunks = std::max(maxChunks, (int)((cells + RED_CHUNK - 1) / RED_CHUNK));
   }
-  h->hPlan.impDoubles = off * 6;
-  h->hPlan.redChunks = maxChunks;
   if (!targets) return LBM_OK;
   int rc = ensure_work(h, std::max(1LL, off * 6), (long long)std::max(ns, 1) * maxChunks * 6);
   if (rc) return rc;
@@ -1905,7 +1903,6 @@ struct lbm_batch {
   long long launches = 0;            // batched fused launches executed
   cudaGraphExec_t exec = nullptr;    // captured 2-step chunk
   std::vector<long long> execKey;    // what it baked in
-  std::vector<long long> execDelta;  // per-scene launches in one chunk
 };
 
 namespace {
@@ -2224,18 +2221,11 @@ int lbm_batch_run(lbm_batch *b, lbm_sphere *const *spheres, const int *nspheres,
     if (!b->exec || key != b->execKey) {
       if (b->exec) cudaGraphExecDestroy(b->exec);
       b->exec = nullptr;
-      std::vector<long long> l0(n);
-      for (int s = 0; s < n; s++) l0[s] = b->sims[s]->launches;
       cudaGraph_t gr = nullptr;
       BCK(cudaStreamBeginCapture(b->origin, cudaStreamCaptureModeThreadLocal));
       int erc = emit_step(0);
       if (erc == LBM_OK) erc = emit_step(1);
       cudaError_t ce = cudaStreamEndCapture(b->origin, &gr);
-      b->execDelta.assign(n, 0);
-      for (int s = 0; s < n; s++) {
-        b->execDelta[s] = b->sims[s]->launches - l0[s];
-        b->sims[s]->launches = l0[s];  // counted when the graph runs
-      }
       if (erc != LBM_OK || ce != cudaSuccess) {
         if (gr) cudaGraphDestroy(gr);
         cudaGetLastError();
@@ -2260,7 +2250,6 @@ int lbm_batch_run(lbm_batch *b, lbm_sphere *const *spheres, const int *nspheres,
   while (done < nsteps) {
     if (graph && nsteps - done >= 2) {
       BCK(cudaGraphLaunch(b->exec, b->origin));
-      for (int s = 0; s < n; s++) b->sims[s]->launches += b->execDelta[s];
       b->launches += 2;
       done += 2;
     } else {

@@ -384,8 +384,6 @@ struct Plan {
   Box U;             // retag / fresh-dead compaction box
   long long ucells;  // cells in U
   int nchunks;       // compaction chunks of U
-  int redChunks;     // impulse-reduction chunks (max over spheres)
-  long long impDoubles;
   Box boxLast, boxLastLast;  // sphere boxes of the two previous retags
   int fullRetag;             // retag the whole grid for this many more steps
   int overflow;              // the plan exceeded the launch capacity

@@ -886,7 +886,6 @@ __device__ __forceinline__ void plan_body(Plan *P, const Plan *prev, const lbm_s
   ss.nsph = nsph;
   ss.zlo = ss.zend = 0;
   Box now{{1, 1, 1}, {0, 0, 0}};
-  int redChunks = 1;
   for (int b = 0; b < nsph; b++) {
     SphereDesc &d = ss.sph[b];
     const double cx = sph[b].cx, cy = sph[b].cy, cz = sph[b].cz, r = sph[b].r;
@@ -915,8 +914,6 @@ __device__ __forceinline__ void plan_body(Plan *P, const Plan *prev, const lbm_s
       t.lo[a] = box_empty(tb) ? 0 : tb.lo[a];
       t.dim[a] = box_empty(tb) ? 0 : tb.hi[a] - tb.lo[a] + 1;
     }
-    const int rc = (int)((cells + RED_CHUNK - 1) / RED_CHUNK);
-    redChunks = rc > redChunks ? rc : redChunks;
   }
   Box U;
   if (fullRetag > 0) {
@@ -938,8 +935,6 @@ __device__ __forceinline__ void plan_body(Plan *P, const Plan *prev, const lbm_s
   P->U = U;
   P->ucells = uc;
   P->nchunks = (int)((uc + COMPACT_CHUNK - 1) / COMPACT_CHUNK);
-  P->redChunks = redChunks;
-  P->impDoubles = (long long)nsph * slotCells * 6;
   P->boxLastLast = boxLast;
   P->boxLast = now;
 }

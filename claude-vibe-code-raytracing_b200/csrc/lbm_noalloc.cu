@@ -42,15 +42,14 @@ constexpr int COMPACT_THREADS = 256;
 
 // Count fresh (FLUID, was SOLID) and dead (SOLID, was FLUID) cells per chunk
 // of the box's linear (scan) order.
-__device__ __forceinline__ void compact_count_body(const uint8_t *tag, const uint8_t *tagPrev, int nx, int ny,
-                                                   const Plan *__restrict__ P, int2 *counts, unsigned bid,
-                                                   unsigned gdim) {
+__global__ void k_compact_count(const uint8_t *tag, const uint8_t *tagPrev, int nx, int ny,
+                                const Plan *__restrict__ P, int2 *counts) {
   __shared__ int sf[COMPACT_THREADS / 32], sd[COMPACT_THREADS / 32];
   const Box bx = P->U;
   const long long total = P->ucells;
   const int nchunks = P->nchunks;
   // CTAs stride over the chunks (block-uniform trip count)
-  for (int c = bid; c < nchunks; c += gdim) {
+  for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
     const long long base = (long long)c * COMPACT_CHUNK;
     int nf = 0, nd = 0;
     for (int j = threadIdx.x; j < COMPACT_CHUNK; j += blockDim.x) {
@@ -83,13 +82,9 @@ __device__ __forceinline__ void compact_count_body(const uint8_t *tag, const uin
     __syncthreads();  // sf / sd are rewritten for the next chunk
   }
 }
-__global__ void k_compact_count(const uint8_t *tag, const uint8_t *tagPrev, int nx, int ny,
-                                       const Plan *__restrict__ P, int2 *counts) {
-  compact_count_body(tag, tagPrev, nx, ny, P, counts, blockIdx.x, gridDim.x);
-}
 
 // Exclusive scan of the per-chunk counts (single CTA, sequential per thread).
-__device__ __forceinline__ void compact_scan_body(int2 *counts, const Plan *__restrict__ P, int *totals) {
+__global__ void k_compact_scan(int2 *counts, const Plan *__restrict__ P, int *totals) {
   __shared__ int2 part[1024];
   const int nchunks = P->nchunks;
   int per = (nchunks + blockDim.x - 1) / blockDim.x;
@@ -121,14 +116,10 @@ __device__ __forceinline__ void compact_scan_body(int2 *counts, const Plan *__re
     run.y += v.y;
   }
 }
-__global__ void k_compact_scan(int2 *counts, const Plan *__restrict__ P, int *totals) {
-  compact_scan_body(counts, P, totals);
-}
 
 // Emit the fresh / dead cell indices in scan order.
-__device__ __forceinline__ void compact_emit_body(const uint8_t *tag, const uint8_t *tagPrev, int nx, int ny,
-                                                  const Plan *__restrict__ P, const int2 *offsets, int *fresh,
-                                                  int *dead, int cap, unsigned bid, unsigned gdim) {
+__global__ void k_compact_emit(const uint8_t *tag, const uint8_t *tagPrev, int nx, int ny,
+                               const Plan *__restrict__ P, const int2 *offsets, int *fresh, int *dead, int cap) {
   __shared__ int wf[COMPACT_THREADS / 32], wd[COMPACT_THREADS / 32];
   __shared__ int runF, runD;
   const Box bx = P->U;
@@ -137,7 +128,7 @@ __device__ __forceinline__ void compact_emit_body(const uint8_t *tag, const uint
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   // CTAs stride over the chunks (block-uniform trip count); the inner loop
   // ends on a barrier, so runF / runD are free to be reset for the next chunk
-  for (int c = bid; c < nchunks; c += gdim) {
+  for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
     const long long base = (long long)c * COMPACT_CHUNK;
     if (threadIdx.x == 0) {
       runF = offsets[c].x;
@@ -189,11 +180,6 @@ __device__ __forceinline__ void compact_emit_body(const uint8_t *tag, const uint
       __syncthreads();
     }
   }
-}
-__global__ void k_compact_emit(const uint8_t *tag, const uint8_t *tagPrev, int nx, int ny,
-                                      const Plan *__restrict__ P, const int2 *offsets, int *fresh,
-                                      int *dead, int cap) {
-  compact_emit_body(tag, tagPrev, nx, ny, P, offsets, fresh, dead, cap, blockIdx.x, gridDim.x);
 }
 
 constexpr long long NOALLOC_MAX_BOX = 1LL << 20;  // cells of the search box
