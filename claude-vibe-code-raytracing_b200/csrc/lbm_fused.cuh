@@ -96,9 +96,9 @@ struct FusedSmem {
 };
 
 // CTAs per SM the register budget is sized for
-// (FP64: as many as its ring leaves room for; sized for three, the kernel kept
-// 96 registers, spilled 680 B a thread and took 267 us a step at 96x80x72,
-// now 224)
+// (FP64: as many as its ring leaves room for; sized for three, the 4-row kernel
+// kept 96 registers, spilled 680 B a thread and took 267 us a step at 96x80x72,
+// now none and 224; 8 rows still spill 24 to 48 B)
 template <class PopT, int TY>
 struct FusedOcc {
   static constexpr int fit = (int)((227 * 1024) / (FusedSmem<PopT, TY>::bytes + 1024));

@@ -11,8 +11,10 @@
 // together, and the cell's coordinates come from 32-bit divisions.  With a
 // rolled loop of scalar accesses and 64-bit divisions ten steps at 112x96x120
 // (FP32, one sphere, the fields read at the end) took 6.19 ms on a B200, now
-// 4.43; the launches now: gradients 8 us, collidePhase 23, streamPhase 18,
-// collideHydro 55 (6.8 TB/s), streamHydroAndMacro 86 (5.1 TB/s).
+// 4.43 to 4.66.  Each phase alone at 256^3 (beyond L2; bytes an interior cell
+// cannot do without): collidePhase 266 us (89 bytes), streamPhase 218 (65),
+// collideHydro 658 (257: 6.4 TB/s, the copy rate is 6.55), streamHydroAndMacro
+// with its impulse read-back 1,026 (297: 4.7 TB/s).
 #pragma once
 
 #include "lbm_fused.cuh"

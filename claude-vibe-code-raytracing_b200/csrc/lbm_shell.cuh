@@ -8,6 +8,9 @@
 // A link needs the cell's own post-collision values; the launch collides the
 // shell's cells once more from the half that the step read, with the tiles'
 // collide_cell, so it gets the same bits without the tiles storing anything.
+// The cells it finishes are those next to a SOLID cell that a sphere of the plan
+// contains; where the tags can hold other SOLID cells a sweep finishes the rest
+// (finish_unowned).
 // Latency-bound: the shells hold 10^2 to 10^4 cells.  What counts is the
 // number of dependent launches and the length of each thread's chain: this one
 // launch takes the place of three (impulse reduction, dead-cell impulses,

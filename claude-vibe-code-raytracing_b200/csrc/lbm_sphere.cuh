@@ -14,7 +14,7 @@ namespace lbm {
 // RigidSphere.step(dt, gravity) (src/solid.js:104-210) in FP64, in the
 // reference's evaluation order: one rounding per operation (round-to-nearest
 // intrinsics on the device; the host side of the library is compiled without
-// FMA contraction).  Shared by the device-resident loop (k_sphere_step) and
+// FMA contraction).  Shared by the device-resident loop (k_shell) and
 // the host entry point lbm_sphere_step_host.
 struct F64 {
   __host__ __device__ static double add(double a, double b) {

@@ -191,7 +191,9 @@ int lbm_step(lbm_sim *sim, const lbm_sphere *spheres, int nspheres, lbm_impulse 
  * scan order when the slabs begin in z order with each slab's two top owned
  * planes copied into the next slab's copied planes after its begin, and the
  * two bottom owned planes copied down before the lower slab's end.
- * lbm_step = begin + end.  LBM_ERR_STATE for a begin after a begin or an end
+ * Fields, tags among them, may be written in between: end takes the tags as
+ * they stand, and SOLID cells that no sphere contains are walls at rest (such a
+ * step costs a whole-grid sweep more).  lbm_step = begin + end.  LBM_ERR_STATE for a begin after a begin or an end
  * without one. */
 int lbm_step_begin(lbm_sim *sim, const lbm_sphere *spheres, int nspheres);
 int lbm_step_end(lbm_sim *sim, const lbm_sphere *spheres, int nspheres, lbm_impulse *out);
