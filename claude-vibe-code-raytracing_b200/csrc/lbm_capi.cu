@@ -341,11 +341,11 @@ void launch_fused(lbm_sim *h, bool anyTag = false) {
   }
 }
 
-// before a fused step: SOLID cells the same in both halves
+// before a fused step: cells that it does not update the same in both halves
 int ready_solid(lbm_sim *h) {
   if (!h->carrySolid) return LBM_OK;
   h->ops->carry_solid(h, 0, h->n);
-  CKL("SOLID cells");
+  CKL("cells at rest");
   h->carrySolid = false;
   return LBM_OK;
 }
@@ -1858,7 +1858,7 @@ int lbm_slab_copy_planes(lbm_sim *dst, int dst_plane, const lbm_sim *src, int sr
   // left to the next step, which does not know them, it swept the whole slab,
   // in every step of a scene of slabs.)
   dst->ops->carry_solid(dst, dc, dc + cells);
-  CKL("SOLID cells of the copied planes");
+  CKL("cells at rest of the copied planes");
   CK(cudaStreamSynchronize(dst->stream));
   dst->listsValid = false;
   dst->tagsOfStep = dst->tagsOfStep && src->tagsOfStep;

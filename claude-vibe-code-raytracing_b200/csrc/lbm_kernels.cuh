@@ -383,11 +383,12 @@ __device__ __forceinline__ void carry_cell(const Scene<PopT, typename Prec<PopT>
     s.uy[nxt][i] = s.uy[cur][i];
   }
 }
-// every SOLID cell of [c0, c1), after calls that may have changed one half alone
+// every cell of [c0, c1) that the step does not update (SOLID, written WALL, the
+// domain's faces), after calls that may have changed one half alone
 template <class PopT>
 __global__ void k_carry_solid(Scene<PopT, typename Prec<PopT>::Real> s, int cur, long long c0, long long c1) {
   for (long long i = c0 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < c1; i += (long long)gridDim.x * blockDim.x)
-    if (s.tag[i] == TAG_SOLID) carry_cell<PopT>(s, cur, i);
+    if (s.tag[i] != TAG_FLUID || !interior_cell(i, s.nx, s.ny, s.nz)) carry_cell<PopT>(s, cur, i);
 }
 
 // ---------------------------------------------------------------- retag, fresh / dead sets, fresh fill

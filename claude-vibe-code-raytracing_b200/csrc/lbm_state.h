@@ -105,7 +105,7 @@ class OpsBase {
   virtual void stream_phase(lbm_sim *h) = 0;
   virtual void collide_hydro(lbm_sim *h) = 0;
   virtual void stream_hydro_macro(lbm_sim *h) = 0;
-  // the SOLID cells of [c0, c1): current half -> the other
+  // the cells of [c0, c1) that a step does not update: current half -> the other
   virtual void carry_solid(lbm_sim *h, long long c0, long long c1) = 0;
   // retag on the plan's box (retag), fresh / dead lists, fresh fill (fill)
   virtual void sets(lbm_sim *h, long long maxChunks, bool retag, bool fill) = 0;
@@ -259,8 +259,9 @@ struct lbm_sim {
   // no tag has been written since the last step's retag (planes copied from
   // another slab of the scene are that slab's)
   bool tagsOfStep = false;
-  // a SOLID cell may differ between the halves (a field write, a phase-by-phase
-  // call): carried over the whole grid before the next fused step
+  // a cell that a step does not update may differ between the halves (a field
+  // write, a phase-by-phase call): carried over the whole grid before the next
+  // fused step
   bool carrySolid = false;
   int fullRetagSteps = 0;
   int nsphLast = 0;
