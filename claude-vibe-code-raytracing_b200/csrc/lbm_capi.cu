@@ -583,7 +583,7 @@ struct CoupledCtx : StepCtx {
 
 // Capacities for the device-computed plan, the plan's history and the device
 // sphere array; everything a captured step needs is allocated here.
-int coupled_prepare(lbm_sim *h, const lbm_sphere *sp, int ns, bool frames, CoupledCtx &c) {
+int coupled_prepare(lbm_sim *h, const lbm_sphere *sp, int ns, int nsteps, bool frames, CoupledCtx &c) {
   int rc = check_spheres(h, sp, ns);
   if (rc) return rc;
   if (h->slab)
@@ -603,7 +603,7 @@ int coupled_prepare(lbm_sim *h, const lbm_sphere *sp, int ns, bool frames, Coupl
   c.redChunks = (int)((c.slotCells + RED_CHUNK - 1) / RED_CHUNK);
   c.tail = true;
   h->tagsOfStep = false;  // (of a step that was begun and not ended)
-  if ((rc = ready_solid(h))) return rc;
+  if (nsteps > 0 && (rc = ready_solid(h))) return rc;
   if ((rc = ensure_work(h, std::max(1LL, (long long)ns * c.slotCells * 6),
                         (long long)std::max(ns, 1) * c.redChunks * 6)))
     return rc;
@@ -1623,7 +1623,7 @@ int lbm_run_coupled(lbm_sim *h, lbm_sphere *sp, int ns, int nsteps, int frame_ev
   if (!h || nsteps < 0) return LBM_ERR_ARG;
   EntryGuard g(h);
   CoupledCtx c;
-  int rc = coupled_prepare(h, sp, ns, frame_every > 0 && frames, c);
+  int rc = coupled_prepare(h, sp, ns, nsteps, frame_every > 0 && frames, c);
   if (rc) return rc;
   long long frame = 0;
   if (nsteps > 0 && (rc = coupled_plan(h, c))) return rc;
@@ -2112,8 +2112,8 @@ int lbm_batch_run(lbm_batch *b, lbm_sphere *const *spheres, const int *nspheres,
   OpsBase *ops = b->sims[0]->ops;
   std::vector<CoupledCtx> ctx(n);
   for (int s = 0; s < n; s++)
-    BSIM(b->sims[s], coupled_prepare(b->sims[s], nspheres[s] ? spheres[s] : nullptr, nspheres[s], wantFrames,
-                                     ctx[s]));
+    BSIM(b->sims[s], coupled_prepare(b->sims[s], nspheres[s] ? spheres[s] : nullptr, nspheres[s], nsteps,
+                                     wantFrames, ctx[s]));
   int rc = batch_tables(b);
   if (rc) return rc;
   // the sparse kernels' arguments of every scene for both parities, and their

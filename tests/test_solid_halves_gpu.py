@@ -114,3 +114,24 @@ def test_a_write_inside_a_split_step(gpu, storage, write):
     for k in FIELDS:
         assert np.array_equal(_cells(sim, k)[rest], want[k]), k
     sim.close()
+
+
+@pytest.mark.parametrize("how", ["run_coupled", "batch"])
+def test_a_run_of_no_steps_changes_nothing(gpu, how):
+    sim, sol = _tank(gpu)
+    for _ in range(3):
+        sim.step(sol)
+    sim.f2[:] = np.float32(0.25)
+    sim.h2[:] = np.float32(0.125)
+    names = FIELDS + ("f2", "h2", "tag", "tagPrev")
+    was = {k: _cells(sim, k) for k in names}
+    state = sol.state()
+    if how == "batch":
+        with gpu.Batch([(sim, sol)]) as batch:
+            batch.run(0)
+    else:
+        sim.run_coupled(sol, 0)
+    for k in names:
+        assert np.array_equal(_cells(sim, k), was[k]), k
+    assert sol.state() == state
+    sim.close()
