@@ -658,6 +658,7 @@ int coupled_finish(lbm_sim *h, lbm_sphere *sp, int ns, int nsteps) {
   h->lastRetagBox = h->hPlan.U;
   h->listsValid = true;
   if (h->hPlan.overflow) {
+    h->hPlan.overflow = 0;  // of this run's plans; the host-driven steps' have room
     h->fullRetagSteps = 2;  // SOLID cells may be left anywhere
     return fail(h, LBM_ERR_CAPACITY, "sphere moved beyond the planned retag box");
   }

@@ -111,3 +111,32 @@ def test_the_next_step_retags_the_whole_grid(gpu, storage):
         for k in STATE:
             assert np.isfinite(np.asarray(getattr(sim, k))).all(), k
     sim.close()
+
+
+@pytest.mark.parametrize("storage", ["f32", "f64"])
+def test_nothing_of_a_run_without_room_is_left_in_later_steps(gpu, storage):
+    """A split step with written tags gives the same bits on a handle with such a
+    run behind it as on a new one."""
+    got = []
+    for failed in (True, False):
+        if failed:
+            sim, sol = _moved(gpu, storage)
+            assert _run(gpu, sim, sol, 2) != 0
+        else:
+            sim = gpu.Sim(*DIMS, storage=storage)
+            scenes._params(sim, 0.8, 0.7, 0.008, 0.0015)
+        sim.initFlat(25)
+        sol = gpu.RigidSphere(*DIMS, cx=30.2, cy=29.8, cz=27.1, r=5.3, density=2.0)
+        rs = np.random.RandomState(5)
+        for k in ("ux", "uy", "uz"):
+            getattr(sim, k)[:] = rs.uniform(-0.05, 0.05, sim.n).astype(np.float32)
+        for _ in range(2):
+            sim.step_begin(sol)
+            tag = np.array(sim.tag).reshape(DIMS[::-1])
+            tag[11, 10, 8:12] = 1  # where the first sphere was
+            sim.tag[:] = tag.ravel()
+            sim.step_end(sol)
+        got.append({k: sim.field64(k) for k in STATE})
+        sim.close()
+    for k in STATE:
+        assert np.array_equal(got[0][k], got[1][k]), k
